@@ -114,6 +114,9 @@ _CUDA_PROTOS = {
     "cvb_router_topk_fwd": "p l iii pp p",
     "cvb_router_topk_bwd": "pppp l iii p p",
     "cvb_expert_layout": "p l ii ppp i pp p",
+    "cvb_moe_dispatch": "ppppp l iii p",
+    "cvb_moe_combine": "pppp l ii p",
+    "cvb_moe_combine_bwd": "pppppppp l iii p",
 }
 
 

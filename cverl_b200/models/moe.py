@@ -71,6 +71,26 @@ def sort_by_expert(expert_ids: torch.Tensor, num_experts: int):
     return order, dest, tile_group.to(torch.int32), offsets.to(torch.int32), m_pad
 
 
+def expert_layout_native(ids: torch.Tensor, num_experts: int, tile_m: int):
+    """``expert_layout`` of contiguous int64 CUDA ids by ``cvb_expert_layout``; the fifth result is int32 [E], the
+    unpadded rows of every expert."""
+    from .. import _native as nv
+    n, dev = ids.numel(), ids.device
+    m_pad = (n + num_experts * (tile_m - 1) + tile_m - 1) // tile_m * tile_m
+    nblocks = (n + 255) // 256
+    scratch = torch.empty(n + (nblocks + 1) * (num_experts + 1), dtype=torch.int32, device=dev)
+    offsets = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)
+    tile_group = torch.empty(m_pad // tile_m, dtype=torch.int32, device=dev)
+    row = torch.empty(n, dtype=torch.int64, device=dev)
+    nv.check(nv.cuda().cvb_expert_layout(ids.data_ptr(), n, num_experts, tile_m, scratch.data_ptr(),
+                                         offsets.data_ptr(), tile_group.data_ptr(), m_pad // tile_m,
+                                         row.data_ptr(), nv.status_word(dev).data_ptr(), nv.stream()),
+             "cvb_expert_layout")
+    ops.launch_counter["n"] += 4
+    totals = scratch[n + nblocks * (num_experts + 1):][:num_experts]
+    return row, tile_group, offsets, m_pad, totals
+
+
 def expert_layout(expert_ids: torch.Tensor, num_experts: int, tile_m: int = TILE_M):
     """``(row, tile_group, offsets, m_pad)``: ``row[i]`` is the row of entry ``i`` in the expert-grouped matrix the
     grouped GEMM reads, every expert's segment padded to a multiple of ``tile_m`` (128) rows and the entries of one
@@ -80,22 +100,8 @@ def expert_layout(expert_ids: torch.Tensor, num_experts: int, tile_m: int = TILE
     from ``sort_by_expert``.  With ``tile_m=1`` it is a plain stable grouping (used for the expert-parallel
     destination rows)."""
     n = expert_ids.numel()
-    dev = expert_ids.device
-    m_pad = (n + num_experts * (tile_m - 1) + tile_m - 1) // tile_m * tile_m
     if expert_ids.is_cuda and expert_ids.dtype == torch.int64 and num_experts <= 256 and n > 0:
-        from .. import _native as nv
-        ids = expert_ids.contiguous()
-        nblocks = (n + 255) // 256
-        scratch = torch.empty(n + (nblocks + 1) * (num_experts + 1), dtype=torch.int32, device=dev)
-        offsets = torch.empty(num_experts + 1, dtype=torch.int32, device=dev)
-        tile_group = torch.empty(m_pad // tile_m, dtype=torch.int32, device=dev)
-        row = torch.empty(n, dtype=torch.int64, device=dev)
-        nv.check(nv.cuda().cvb_expert_layout(ids.data_ptr(), n, num_experts, tile_m, scratch.data_ptr(),
-                                             offsets.data_ptr(), tile_group.data_ptr(), m_pad // tile_m,
-                                             row.data_ptr(), nv.status_word(dev).data_ptr(), nv.stream()),
-                 "cvb_expert_layout")
-        ops.launch_counter["n"] += 4
-        return row, tile_group, offsets, m_pad
+        return expert_layout_native(expert_ids.contiguous(), num_experts, tile_m)[:4]
     if tile_m != TILE_M:
         raise ValueError("the tensor-op layout pads to 128 rows only")
     order, dest, tile_group, offsets, m_pad = sort_by_expert(expert_ids, num_experts)
@@ -129,6 +135,10 @@ def moe_mlp(model, x: torch.Tensor, layer: int) -> torch.Tensor:
     # paths over the group), and the gate matrix is one of ``tp_partial_grad_names``.
     x_in = copy_to_tp(x, ctx.tp_group)
     idx, w = router(x_in, model.param(p + "gate.weight"), k, cfg.norm_topk_prob)
+    if ctx.ep_size == 1:
+        from ..ops.moe import moe_experts, supported
+        if supported(x_in, gate_up, down, k):
+            return reduce_from_tp(moe_experts(x_in, idx, w, gate_up, down), ctx.tp_group)
     rows = x_in.repeat_interleave(k, dim=0)                              # one row per (token, k) pair
     flat_e = idx.reshape(-1)
     if ctx.ep_size == 1:
