@@ -1,39 +1,51 @@
-// Causal / blockwise GQA attention on tcgen05 (head dim 128 or 256), forward pass.
+// Causal / blockwise GQA attention on tcgen05 (head dim 128 or 256), forward and backward.
 //
-// One CTA per (128-query block, query head, batch).  Q stays in shared memory; K / V stream through two
-// TMA buffers in blocks of 64 keys.  Per key block:
-//     S  = Q K^T            tcgen05 MMA, M = 128, N = 64, K = D         -> TMEM
-//     P  = exp2(S c - m)    one thread per query row (a TMEM lane is a row: no shuffles), running max m
-//                           and sum l in registers, bf16 P written to shared memory
-//     O += P V              tcgen05 MMA, M = 128, N = D, K = 64, V read MN-major from the TMA tile
-// The accumulator O lives in TMEM for the whole CTA; it is rescaled only when a row's maximum has grown
-// by more than 2^8 since the last rescale (the stale maximum keeps P <= 256, exactness is kept because
-// l uses the same maximum).  Query / key position offsets make the same kernel serve the hops of
-// context-parallel ring attention: it returns the un-merged (O, LSE) of one key range.
+// Forward: a CTA owns NT tiles of 128 queries of one head (NT = 1 at head dim 256, 2 at 128: with S and O of NT
+// tiles tensor memory is full either way) and walks the keys in blocks of 128.
+//     S  = Q K^T            tcgen05 MMA, M = 128, N = 128, K = D         -> TMEM
+//     P  = exp2(S c - m)    one thread per query row (a TMEM lane is a row: no shuffles), running max m and sum l in
+//                           registers; bf16 P goes back to TMEM over the columns of S it came from
+//     O += P V              tcgen05 MMA, A = P from TMEM, N = D, V read MN-major from the TMA tile
+// Roles: warp 0 streams K and V through a ring of five 32 KB stages, warp 1 issues the MMAs, warps 4-7 (and 8-11)
+// do the softmax of tile 0 (and 1).  The tensor cores work on one S slot while the softmax works on the other: at
+// NT = 1 the slots alternate by key block (S of block j + 1 is issued before O += P V of block j), at NT = 2 each
+// tile has its own.  MMAs of one CTA retire in issue order, so a slot is overwritten by the next S only after its P
+// has been read, without a wait.
+// The accumulator O is rescaled only when a row's maximum has grown by more than 2^8 since the last rescale (the
+// stale maximum keeps P <= 256, exactness is kept because l uses the same maximum).  Query / key position offsets
+// make the same kernel serve the hops of context-parallel ring attention: it returns the un-merged (O, LSE) of one
+// key range.  Sequences of any length: rows past the end are zero-filled by TMA, masked as keys and clipped by the
+// TMA store as queries.
+// Bound by the tensor cores at head dim 256 and by the exponentials at 128.
+// Causal, 16 x 1280 with 8 query and 2 kv heads of 256: 148 us (727 TFLOP/s), 269 us as one serial chain per CTA in
+// blocks of 64 keys.  1 x 8192 of the same heads runs at 1,302 TFLOP/s, 2 x 4096 with 32 heads of 128 at 941: at
+// 1280 what remains is the fill and drain of each CTA's chain of 5.5 blocks on average.
 //
 // The reference calls at::scaled_dot_product_attention (src/model/qwen3_5_text.cc:1068-1075) and, for
 // context parallelism, a scalar SIMT kernel (cuda/cp_attention_cuda.cu).
 #include "ptx.cuh"
 #include "gemm_tcgen05.h"
+#include <initializer_list>
 
 namespace cvb {
 
-constexpr int AT_THREADS = 128;
-constexpr int AT_BQ = 128;   // queries per CTA
-constexpr int AT_BK = 64;    // keys per block
+constexpr int AT_BQ = 128;       // queries per tile
+constexpr int AT_BK = 128;       // keys per block
+constexpr int AT_STAGES = 5;
+constexpr int AT_STAGE = 32768;  // bytes of a stage: a K or V block at head dim 128, half a block at 256
 
 template <int D>
-struct AttSmem {
-  static constexpr int Q = 0;                       // D/64 boxes [128 x 64]
-  static constexpr int K = D * 256;                 // 2 buffers x D/64 boxes [64 x 64]
-  static constexpr int V = K + 2 * D * 128;
-  static constexpr int P = V + 2 * D * 128;         // [128 x 64] bf16
-  static constexpr int BARS = P + 16384;
+struct AttCfg {
+  static constexpr int NT = 256 / D;                // query tiles per CTA
+  static constexpr int PER = D / 128;               // stages per K or V block
+  static constexpr int THREADS = 128 + 128 * NT;
+  static constexpr int Q = 0;                       // NT tiles of D/64 boxes [128 x 64]
+  static constexpr int RING = 65536;
+  static constexpr int BARS = RING + AT_STAGES * AT_STAGE;
   static constexpr int BYTES = BARS + 256 + 1024;
 };
 
 struct AttArgs {
-  __nv_bfloat16* out;   // [B, Sq, Hq, D]
   float* lse;           // [B, Hq, Sq]  natural-log LSE of the scaled scores (-inf for a fully masked row)
   int Sq, Skv, Hq, Hkv, B;
   float scale_log2;     // softmax scale * log2(e)
@@ -47,230 +59,370 @@ __device__ __forceinline__ uint32_t asw128(uint32_t row, uint32_t chunk) {
 }
 
 template <int D>
-__global__ void __launch_bounds__(AT_THREADS, 1)
+__global__ void __launch_bounds__(AttCfg<D>::THREADS, 1)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                     const __grid_constant__ CUtensorMap tmV, const AttArgs a) {
-  using SM = AttSmem<D>;
-  constexpr int NB = D / 64;            // 64-column boxes per row
-  constexpr uint32_t KV_BYTES = 2u * D * 128u;  // one K block + one V block
-  constexpr uint32_t TCOLS = (D == 256) ? 512 : 256;  // S (64) + O (D), rounded up to a power of two
+                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
+                     const AttArgs a) {
+  using C = AttCfg<D>;
+  constexpr int NT = C::NT, PER = C::PER, NB = D / 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::BARS);
-  uint64_t *bar_q = bars, *bar_kv = bars + 1 /* [2] */, *bar_s = bars + 3, *bar_o = bars + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::BARS);
+  uint64_t* bar_q = bars;
+  uint64_t* bar_full = bars + 1;                 // [AT_STAGES]
+  uint64_t* bar_empty = bar_full + AT_STAGES;    // [AT_STAGES]
+  uint64_t* bar_s = bar_empty + AT_STAGES;       // [2] S of a slot is complete
+  uint64_t* bar_p = bar_s + 2;                   // [2] P of a slot is in TMEM, O is rescaled
+  uint64_t* bar_o = bar_p + 2;                   // [NT] O += P V of a tile is complete
+  uint64_t* bar_out = bar_o + 2;                 // [NT] the tile's output is staged
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_out + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // 1-D grid, last query block first: under the causal mask it sees the most keys, so the longest CTAs are
   // scheduled first and the launch ends with short ones.
   const int per_block = a.Hq * a.B;
-  const int q0 = (a.Sq / AT_BQ - 1 - static_cast<int>(blockIdx.x / per_block)) * AT_BQ;
+  const int q_blocks = (a.Sq + NT * AT_BQ - 1) / (NT * AT_BQ);
+  const int q0 = (q_blocks - 1 - static_cast<int>(blockIdx.x / per_block)) * (NT * AT_BQ);
   const int h = (blockIdx.x % per_block) % a.Hq;
   const int hk = h / (a.Hq / a.Hkv);
-  const long long b = (blockIdx.x % per_block) / a.Hq;
+  const int b = (blockIdx.x % per_block) / a.Hq;
   const uint32_t sb = smem_u32(smem);
 
-  // key blocks this query block can see
-  int nblk = a.Skv / AT_BK;
-  if (a.causal) {
-    const long long last_q = a.q_pos0 + q0 + AT_BQ - 1;
-    const long long lim = last_q - a.k_pos0;         // largest visible key index
-    nblk = lim < 0 ? 0 : static_cast<int>(min(static_cast<long long>(nblk), lim / AT_BK + 1));
-  }
-
-  auto load_kv = [&](int j) {
-    const int buf = j & 1;
-    const int krow = static_cast<int>(b * a.Skv + static_cast<long long>(j) * AT_BK);
-    mbar_arrive_expect_tx(&bar_kv[buf], KV_BYTES);
+  // key blocks that each tile can see
+  int n[NT], nmax = 0;
 #pragma unroll
-    for (int c = 0; c < NB; ++c) {
-      tma_load_2d(smem + SM::K + buf * (D * 128) + c * 8192, &tmK, &bar_kv[buf], hk * D + c * 64, krow);
-      tma_load_2d(smem + SM::V + buf * (D * 128) + c * 8192, &tmV, &bar_kv[buf], hk * D + c * 64, krow);
+  for (int t = 0; t < NT; ++t) {
+    const int first = q0 + t * AT_BQ;
+    int k = (a.Skv + AT_BK - 1) / AT_BK;
+    if (a.causal) {
+      const long long lim = a.q_pos0 + min(first + AT_BQ, a.Sq) - 1 - a.k_pos0;   // largest visible key index
+      k = lim < 0 ? 0 : static_cast<int>(min(static_cast<long long>(k), lim / AT_BK + 1));
     }
-  };
+    n[t] = first < a.Sq ? k : 0;
+    nmax = max(nmax, n[t]);
+  }
 
   if (tid == 0) {
-    mbar_init(bar_q, 1); mbar_init(&bar_kv[0], 1); mbar_init(&bar_kv[1], 1); mbar_init(bar_s, 1); mbar_init(bar_o, 1);
+    mbar_init(bar_q, 1);
+    for (int s = 0; s < AT_STAGES; ++s) {
+      mbar_init(&bar_full[s], 1);
+      mbar_init(&bar_empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&bar_s[s], 1);
+      mbar_init(&bar_p[s], 4);   // one arrival per softmax warp
+      mbar_init(&bar_o[s], 1);
+      mbar_init(&bar_out[s], 4);
+    }
     *abort_flag = 0;
     mbar_fence_init();
-    if (nblk > 0) {
-      mbar_arrive_expect_tx(bar_q, D * 256);
-      const int qrow = static_cast<int>(b * a.Sq + q0);
-#pragma unroll
-      for (int c = 0; c < NB; ++c) tma_load_2d(smem + SM::Q + c * 16384, &tmQ, bar_q, h * D + c * 64, qrow);
-      load_kv(0);
-      if (nblk > 1) load_kv(1);
-    }
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
   }
-  if (warp == 0) {
-    __syncwarp();
-    tmem_alloc(tmem_slot, TCOLS);
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
-  constexpr uint32_t TC_S = 0, TC_O = 64;
+  constexpr uint32_t TC_S = 0, TC_O = 256;   // S slot s at 128 s, O of tile t at 256 + t D
 
-  float m = -INFINITY, m_used = -INFINITY, l = 0.f;
-  const long long qpos = a.q_pos0 + q0 + tid;
-  bool ok = true;
-  if (nblk > 0) {
-    if (!mbar_wait_bounded(bar_q, 0, abort_flag)) {
-      if (!*abort_flag) atomicCAS(a.status, 0, ERR_WAIT_FULL);
-      *abort_flag = 1;
+  auto fail = [&](int code) {
+    if (!*abort_flag) atomicCAS(a.status, 0, code);
+    *abort_flag = 1;
+  };
+
+  if (warp == 0) {
+    // ------------------------------ TMA producer ------------------------------
+    if (lane == 0 && nmax > 0) {
+      mbar_arrive_expect_tx(bar_q, NT * D * 256);
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int c = 0; c < NB; ++c)
+          tma_load_3d(smem + C::Q + (t * NB + c) * 16384, &tmQ, bar_q, h * D + c * 64, q0 + t * AT_BQ, b);
+      int stage = 0;
+      uint32_t phase = 0, armed = 0, parity = 0;
+      bool ok = true;
+      auto load = [&](int j, bool is_k) {
+        for (int hf = 0; hf < PER && ok; ++hf) {
+          if (!mbar_wait_bounded(&bar_empty[stage], phase ^ 1, abort_flag)) {
+            fail(ERR_WAIT_EMPTY);
+            ok = false;
+            break;
+          }
+          uint8_t* dst = smem + C::RING + stage * AT_STAGE;
+          mbar_arrive_expect_tx(&bar_full[stage], AT_STAGE);
+          if (is_k) {   // 128 keys x 128 columns
+            for (int c = 0; c < 2; ++c)
+              tma_load_3d(dst + c * 16384, &tmK, &bar_full[stage], hk * D + hf * 128 + c * 64, j * AT_BK, b);
+          } else {      // head dim 128: 128 keys x 128 columns; 256: 64 keys x 256 columns
+            constexpr int KEYS = AT_BK / PER;
+            for (int c = 0; c < NB; ++c)
+              tma_load_3d(dst + c * (KEYS * 128), &tmV, &bar_full[stage], hk * D + c * 64, j * AT_BK + hf * KEYS, b);
+          }
+          armed |= 1u << stage;
+          parity = (parity & ~(1u << stage)) | (phase << stage);
+          if (++stage == AT_STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      };
+      load(0, true);
+      for (int j = 0; j < nmax && ok; ++j) {   // in the order in which the MMA warp takes them
+        if (NT == 1) {
+          if (j + 1 < nmax) load(j + 1, true);
+          load(j, false);
+        } else {
+          load(j, false);
+          if (j + 1 < nmax) load(j + 1, true);
+        }
+      }
+      if (!ok || *abort_flag) {   // leave no copy in flight
+        int dummy = 0;
+        mbar_wait_bounded(bar_q, 0, &dummy);
+        for (int s = 0; s < AT_STAGES; ++s)
+          if (armed & (1u << s)) mbar_wait_bounded(&bar_full[s], (parity >> s) & 1, &dummy);
+      }
     }
-    __syncthreads();
-    ok = !*abort_flag;
-  }
-  for (int j = 0; j < nblk && ok; ++j) {
-    const int buf = j & 1;
-    const uint32_t ph = (j >> 1) & 1, pj = j & 1;
-    // ---- S = Q K^T -------------------------------------------------------------------------------------
-    if (tid == 0) {
-      if (mbar_wait_bounded(&bar_kv[buf], ph, abort_flag)) {
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer --------------------------------
+    if (lane == 0 && nmax > 0) {
+      constexpr uint32_t id_s = umma_idesc(128, AT_BK, 1, 0, 0);
+      constexpr uint32_t id_o = umma_idesc(128, D, 1, 0, 1);
+      bool ok = mbar_wait_bounded(bar_q, 0, abort_flag);
+      if (!ok) fail(ERR_WAIT_FULL);
+      int stage = 0;          // next stage of the ring, in the producer's order
+      uint32_t phase = 0;
+      auto take = [&]() {     // waits for the next stage; returns its index
+        const int s = stage;
+        if (ok && !mbar_wait_bounded(&bar_full[s], phase, abort_flag)) {
+          fail(ERR_WAIT_FULL);
+          ok = false;
+        }
+        if (++stage == AT_STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
+        return s;
+      };
+      auto qk = [&](int t, int slot, const int (&st)[2]) {
         tc_fence_after();
-        constexpr uint32_t idesc = umma_idesc(128, AT_BK, 1, 0, 0);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t kb = k >> 2, ks = (k & 3) * 32;
-          umma_bf16(tmem_base + TC_S, umma_smem_desc(sb + SM::Q + kb * 16384 + ks, 16, 1024),
-                    umma_smem_desc(sb + SM::K + buf * (D * 128) + kb * 8192 + ks, 16, 1024), idesc, k > 0);
+          umma_bf16(tmem_base + TC_S + slot * 128, umma_smem_desc(sb + C::Q + (t * NB + kb) * 16384 + ks, 16, 1024),
+                    umma_smem_desc(sb + C::RING + st[kb >> 1] * AT_STAGE + (kb & 1) * 16384 + ks, 16, 1024), id_s,
+                    k > 0);
         }
-        umma_commit(bar_s);
-      } else {
-        if (!*abort_flag) atomicCAS(a.status, 0, ERR_WAIT_FULL);
-        *abort_flag = 1;
-      }
-    }
-    if (!mbar_wait_bounded(bar_s, pj, abort_flag)) {
-      if (!*abort_flag) atomicCAS(a.status, 0, ERR_WAIT_TMEM_FULL);
-      *abort_flag = 1;
-    }
-    __syncthreads();
-    if (*abort_flag) { ok = false; break; }
-    tc_fence_after();
-    // ---- softmax of this block, one row per thread -------------------------------------------------------
-    {
-      uint32_t r0[32], r1[32];
-      tmem_ld_32x32(tmem + TC_S, r0);
-      tmem_ld_32x32(tmem + TC_S + 32, r1);
-      tmem_ld_wait();
-      const long long kbase = a.k_pos0 + static_cast<long long>(j) * AT_BK;
-      const bool diag = a.causal && (kbase + AT_BK - 1 > a.q_pos0 + q0);
-      // number of visible keys of this row in the block
-      int vis = AT_BK;
-      if (diag) {
-        const long long v64 = qpos - kbase + 1;
-        vis = v64 < 0 ? 0 : (v64 > AT_BK ? AT_BK : static_cast<int>(v64));
-      }
-      float mx = -INFINITY;
+        umma_commit(&bar_s[slot]);
+      };
+      auto pv = [&](int t, int slot, const int (&st)[2], bool first, bool last_use) {
+        tc_fence_after();
+        constexpr int KEYS = AT_BK / PER;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        if (i < vis) mx = fmaxf(mx, __uint_as_float(r0[i]));
-        if (32 + i < vis) mx = fmaxf(mx, __uint_as_float(r1[i]));
+        for (int hf = 0; hf < PER; ++hf) {
+#pragma unroll
+          for (int k = 0; k < KEYS / 16; ++k)
+            umma_bf16_ts(tmem_base + TC_O + t * D, tmem_base + TC_S + slot * 128 + (hf * (KEYS / 16) + k) * 8,
+                         umma_smem_desc(sb + C::RING + st[hf] * AT_STAGE + k * 2048, KEYS * 128, 1024), id_o,
+                         !(first && hf == 0 && k == 0));
+          if (last_use) umma_commit(&bar_empty[st[hf]]);
+        }
+        umma_commit(&bar_o[t]);
+      };
+      auto wait_p = [&](int slot, uint32_t par) {
+        if (ok && !mbar_wait_bounded(&bar_p[slot], par, abort_flag)) {
+          fail(ERR_WAIT_TMEM_EMPTY);
+          ok = false;
+        }
+      };
+      int ks[2] = {0, 0}, vs[2] = {0, 0};
+      for (int i = 0; i < PER; ++i) ks[i] = take();
+      if (ok) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+          if (n[t] > 0) qk(t, t, ks);
+        for (int i = 0; i < PER; ++i) umma_commit(&bar_empty[ks[i]]);
       }
-      mx *= a.scale_log2;   // scale > 0
-      m = fmaxf(m, mx);
+      for (int j = 0; j < nmax && ok; ++j) {
+        if (NT == 1) {
+          const int slot = j & 1;
+          if (j + 1 < nmax) {
+            for (int i = 0; i < PER; ++i) ks[i] = take();
+            if (!ok) break;
+            qk(0, slot ^ 1, ks);
+            for (int i = 0; i < PER; ++i) umma_commit(&bar_empty[ks[i]]);
+          }
+          for (int i = 0; i < PER; ++i) vs[i] = take();
+          wait_p(slot, (j >> 1) & 1);
+          if (!ok) break;
+          pv(0, slot, vs, j == 0, true);
+        } else {
+          vs[0] = take();
+          if (j + 1 < nmax) ks[0] = take();
+          if (!ok) break;
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            if (j < n[t]) {
+              wait_p(t, j & 1);
+              if (!ok) break;
+              pv(t, t, vs, j == 0, false);
+              if (j + 1 < n[t]) qk(t, t, ks);
+            }
+          }
+          if (!ok) break;
+          umma_commit(&bar_empty[vs[0]]);
+          if (j + 1 < nmax) umma_commit(&bar_empty[ks[0]]);
+        }
+      }
+    }
+  } else if (warp >= 4) {
+    // ------------------------------ softmax, one row per thread ---------------
+    const int t = NT == 1 ? 0 : (warp >> 2) - 1;
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t tmem = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const uint32_t t_o = tmem + TC_O + t * D;
+    const int qi = q0 + t * AT_BQ + row;
+    const long long qpos = a.q_pos0 + qi;
+    const long long first_pos = a.q_pos0 + q0 + t * AT_BQ;
+    const int nt = t == 0 ? n[0] : n[NT - 1];
+    float m_used = -INFINITY, m = -INFINITY, l = 0.f;
+    bool ok = true;
+    for (int j = 0; j < nt; ++j) {
+      const int slot = NT == 1 ? (j & 1) : t;
+      const uint32_t par = NT == 1 ? (j >> 1) & 1 : j & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_s[slot], par, abort_flag));
+      if (!ok) {
+        if (lane == 0) fail(ERR_WAIT_TMEM_FULL);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t t_s = tmem + TC_S + slot * 128;
+      uint32_t r[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + c * 32, r[c]);
+      tmem_ld_wait();
+      const int k0 = j * AT_BK;
+      // only the blocks on the diagonal and the last one hold keys that some row must not see
+      if (k0 + AT_BK > a.Skv || (a.causal && a.k_pos0 + k0 + AT_BK - 1 > first_pos)) {
+        long long vis64 = a.Skv - k0;
+        if (a.causal) vis64 = min(vis64, qpos - (a.k_pos0 + k0) + 1);
+        const int vis = static_cast<int>(max(min(vis64, static_cast<long long>(AT_BK)), 0ll));
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i >= vis) r[c][i] = __float_as_uint(-INFINITY);
+      }
+      float mx[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        mx[c] = __uint_as_float(r[c][0]);
+#pragma unroll
+        for (int i = 1; i < 32; ++i) mx[c] = fmaxf(mx[c], __uint_as_float(r[c][i]));
+      }
+      m = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.scale_log2);   // scale > 0
       const bool want = (m > m_used + 8.f) || (m_used == -INFINITY && m > -INFINITY);
       if (__any_sync(0xffffffffu, want)) {   // warp-uniform: tcgen05.ld / st are warp-collective
         const float alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - m);
         m_used = m;
         l *= alpha;
         if (j > 0) {
+          ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_o[t], (j - 1) & 1, abort_flag));
+          if (!ok) {
+            if (lane == 0) fail(ERR_WAIT_TMEM_FULL);
+            break;
+          }
+          tc_fence_after();
 #pragma unroll 1
-          for (int c0 = 0; c0 < D; c0 += 32) {
-            uint32_t o[32];
-            tmem_ld_32x32(tmem + TC_O + c0, o);
+          for (int c0 = 0; c0 < D; c0 += 16) {
+            uint32_t o[16];
+            tmem_ld_32x16(t_o + c0, o);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32(tmem + TC_O + c0, o);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x16(t_o + c0, o);
           }
-          tmem_st_wait();
         }
       }
-      float p[64];
-      float sum = 0.f;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        p[i] = (i < vis) ? exp2f(__uint_as_float(r0[i]) * a.scale_log2 - m_used) : 0.f;
-        p[32 + i] = (32 + i < vis) ? exp2f(__uint_as_float(r1[i]) * a.scale_log2 - m_used) : 0.f;
-        sum += p[i] + p[32 + i];
-      }
-      l += sum;
-      uint8_t* prow = smem + SM::P;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint4 u;
-        u.x = pack_bf16x2(p[8 * c + 0], p[8 * c + 1]);
-        u.y = pack_bf16x2(p[8 * c + 2], p[8 * c + 3]);
-        u.z = pack_bf16x2(p[8 * c + 4], p[8 * c + 5]);
-        u.w = pack_bf16x2(p[8 * c + 6], p[8 * c + 7]);
-        *reinterpret_cast<uint4*>(prow + asw128(tid, c)) = u;
-      }
-    }
-    fence_proxy_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    // ---- O += P V ----------------------------------------------------------------------------------------
-    if (tid == 0) {
-      constexpr uint32_t idesc = umma_idesc(128, D, 1, 0, 1);
-#pragma unroll
-      for (int k = 0; k < AT_BK / 16; ++k)
-        umma_bf16(tmem_base + TC_O, umma_smem_desc(sb + SM::P + k * 32, 16, 1024),
-                  umma_smem_desc(sb + SM::V + buf * (D * 128) + k * 2048, 8192, 1024), idesc, (j > 0 || k > 0));
-      umma_commit(bar_o);
-    }
-    if (!mbar_wait_bounded(bar_o, pj, abort_flag)) {
-      if (!*abort_flag) atomicCAS(a.status, 0, ERR_WAIT_TMEM_FULL);
-      *abort_flag = 1;
-    }
-    __syncthreads();
-    if (*abort_flag) { ok = false; break; }
-    tc_fence_after();
-    if (tid == 0 && j + 2 < nblk) load_kv(j + 2);   // this buffer is free again
-  }
-  if (!ok && tid == 0) {   // leave no copy in flight
-    int dummy = 0;
-    mbar_wait_bounded(&bar_kv[0], 0, &dummy);
-    mbar_wait_bounded(&bar_kv[1], 0, &dummy);
-  }
-  if (ok) {
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    __nv_bfloat16* orow = a.out + ((b * a.Sq + q0 + tid) * a.Hq + h) * D;
-#pragma unroll 1
-    for (int c0 = 0; c0 < D; c0 += 32) {
-      uint32_t o[32];
-      if (nblk > 0) {
-        tmem_ld_32x32(tmem + TC_O + c0, o);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] = 0u;
-      }
+      const float mm = m_used == -INFINITY ? 0.f : m_used;
+      float sum[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        uint4 u;
-        u.x = pack_bf16x2(__uint_as_float(o[8 * c + 0]) * inv, __uint_as_float(o[8 * c + 1]) * inv);
-        u.y = pack_bf16x2(__uint_as_float(o[8 * c + 2]) * inv, __uint_as_float(o[8 * c + 3]) * inv);
-        u.z = pack_bf16x2(__uint_as_float(o[8 * c + 4]) * inv, __uint_as_float(o[8 * c + 5]) * inv);
-        u.w = pack_bf16x2(__uint_as_float(o[8 * c + 6]) * inv, __uint_as_float(o[8 * c + 7]) * inv);
-        *reinterpret_cast<uint4*>(orow + c0 + 8 * c) = u;
+        uint32_t p[16];
+        sum[c] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float p0 = exp2f(__uint_as_float(r[c][2 * i]) * a.scale_log2 - mm);
+          const float p1 = exp2f(__uint_as_float(r[c][2 * i + 1]) * a.scale_log2 - mm);
+          sum[c] += p0 + p1;
+          p[i] = pack_bf16x2(p0, p1);
+        }
+        tmem_st_32x16(t_s + c * 16, p);
+      }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_p[slot]);
+    }
+    if (ok && nmax > 0) {   // a tile without visible keys still waits for its Q, whose place the output takes
+      ok = __all_sync(0xffffffffu, nt > 0 ? mbar_wait_bounded(&bar_o[t], (nt - 1) & 1, abort_flag)
+                                          : mbar_wait_bounded(bar_q, 0, abort_flag));
+      if (!ok && lane == 0) fail(ERR_WAIT_TMEM_FULL);
+    }
+    if (ok && q0 + t * AT_BQ < a.Sq) {
+      tc_fence_after();
+      // O / l as bf16 over this tile's Q (its last S is complete), then out by TMA, which drops rows past the end
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      uint8_t* stage = smem + C::Q + t * (D * 256);
+#pragma unroll 1
+      for (int c0 = 0; c0 < D; c0 += 32) {
+        uint32_t o[32];
+        if (nt > 0) {
+          tmem_ld_32x32(t_o + c0, o);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = 0u;
+        }
+        uint8_t* box = stage + (c0 >> 6) * 16384;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint4 u;
+          u.x = pack_bf16x2(__uint_as_float(o[8 * c + 0]) * inv, __uint_as_float(o[8 * c + 1]) * inv);
+          u.y = pack_bf16x2(__uint_as_float(o[8 * c + 2]) * inv, __uint_as_float(o[8 * c + 3]) * inv);
+          u.z = pack_bf16x2(__uint_as_float(o[8 * c + 4]) * inv, __uint_as_float(o[8 * c + 5]) * inv);
+          u.w = pack_bf16x2(__uint_as_float(o[8 * c + 6]) * inv, __uint_as_float(o[8 * c + 7]) * inv);
+          *reinterpret_cast<uint4*>(box + asw128(row, ((c0 & 32) >> 3) + c)) = u;
+        }
+      }
+      if (qi < a.Sq)
+        a.lse[(static_cast<long long>(b) * a.Hq + h) * a.Sq + qi] =
+            l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_out[t]);
+      if (row == 0 && mbar_wait_bounded(&bar_out[t], 0, abort_flag)) {
+#pragma unroll
+        for (int c = 0; c < NB; ++c)
+          tma_store_3d(&tmO, stage + c * 16384, h * D + c * 64, q0 + t * AT_BQ, b);
+        tma_store_commit();
+        tma_store_wait_all();
       }
     }
-    a.lse[(b * a.Hq + h) * a.Sq + q0 + tid] = l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
+  if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TCOLS);
+    tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -278,25 +430,29 @@ template <int D>
 static int launch_fwd(const void* q, const void* k, const void* v, void* out, float* lse, long long B, int Sq,
                       int Skv, int Hq, int Hkv, float scale, int causal, long long q_pos0, long long k_pos0,
                       int* status, cudaStream_t st) {
-  CUtensorMap mq, mk, mv;
-  if (make_tensor_map_2d(&mq, q, 2, static_cast<uint64_t>(Hq) * D, B * Sq, static_cast<uint64_t>(Hq) * D * 2, 64, 128) ||
-      make_tensor_map_2d(&mk, k, 2, static_cast<uint64_t>(Hkv) * D, B * Skv, static_cast<uint64_t>(Hkv) * D * 2, 64, 64) ||
-      make_tensor_map_2d(&mv, v, 2, static_cast<uint64_t>(Hkv) * D, B * Skv, static_cast<uint64_t>(Hkv) * D * 2, 64, 64))
+  using C = AttCfg<D>;
+  CUtensorMap mq, mk, mv, mo;
+  const uint64_t qc = static_cast<uint64_t>(Hq) * D, kc = static_cast<uint64_t>(Hkv) * D;
+  if (make_tensor_map_3d(&mq, q, 2, qc, Sq, B, qc * 2, qc * 2 * Sq, 64, AT_BQ) ||
+      make_tensor_map_3d(&mo, out, 2, qc, Sq, B, qc * 2, qc * 2 * Sq, 64, AT_BQ) ||
+      make_tensor_map_3d(&mk, k, 2, kc, Skv, B, kc * 2, kc * 2 * Skv, 64, AT_BK) ||
+      make_tensor_map_3d(&mv, v, 2, kc, Skv, B, kc * 2, kc * 2 * Skv, 64, AT_BK / C::PER))
     return -10;
   AttArgs a{};
-  a.out = static_cast<__nv_bfloat16*>(out); a.lse = lse; a.Sq = Sq; a.Skv = Skv; a.Hq = Hq; a.Hkv = Hkv;
+  a.lse = lse; a.Sq = Sq; a.Skv = Skv; a.Hq = Hq; a.Hkv = Hkv;
   a.B = static_cast<int>(B);
   a.scale_log2 = scale * 1.4426950408889634f; a.causal = causal; a.q_pos0 = q_pos0; a.k_pos0 = k_pos0;
   a.status = status;
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(attention_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             AttSmem<D>::BYTES) != cudaSuccess)
+    if (cudaFuncSetAttribute(attention_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::BYTES) !=
+        cudaSuccess)
       return -11;
     attr = true;
   }
-  dim3 grid(static_cast<unsigned>((Sq / AT_BQ) * Hq * B));
-  attention_fwd_kernel<D><<<grid, AT_THREADS, AttSmem<D>::BYTES, st>>>(mq, mk, mv, a);
+  const long long blocks = static_cast<long long>((Sq + C::NT * AT_BQ - 1) / (C::NT * AT_BQ)) * Hq * B;
+  if (blocks > 0x7fffffffLL) return -2;
+  attention_fwd_kernel<D><<<static_cast<unsigned>(blocks), C::THREADS, C::BYTES, st>>>(mq, mk, mv, mo, a);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -305,14 +461,16 @@ static int launch_fwd(const void* q, const void* k, const void* v, void* out, fl
 using namespace cvb;
 
 // q: bf16 [B, Sq, Hq, D]; k, v: bf16 [B, Skv, Hkv, D] (all contiguous); out: bf16 [B, Sq, Hq, D];
-// lse: fp32 [B, Hq, Sq].  D in {128, 256}; Sq % 128 == 0; Skv % 64 == 0; Hq % Hkv == 0.
+// lse: fp32 [B, Hq, Sq].  D in {128, 256}; Hq % Hkv == 0; any Sq and Skv.
 // causal != 0 masks keys whose position (k_pos0 + index) exceeds the query's (q_pos0 + index).
 extern "C" int cvb_attention_fwd(const void* q, const void* k, const void* v, void* out, float* lse, long long B,
                                  int Sq, int Skv, int Hq, int Hkv, int D, float scale, int causal, long long q_pos0,
                                  long long k_pos0, int* status, void* stream) {
   if (B <= 0 || Sq <= 0 || Skv <= 0) return 0;
-  if (Sq % AT_BQ || Skv % AT_BK || Hkv <= 0 || Hq % Hkv || !(scale > 0.f)) return -1;
+  if (Hkv <= 0 || Hq % Hkv || !(scale > 0.f)) return -1;
   if (B * Sq > 0x7fffffffLL || B * Skv > 0x7fffffffLL) return -2;
+  for (const void* p : {q, k, v, static_cast<const void*>(out)})
+    if (reinterpret_cast<uintptr_t>(p) & 15) return -3;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (D == 128) return launch_fwd<128>(q, k, v, out, lse, B, Sq, Skv, Hq, Hkv, scale, causal, q_pos0, k_pos0, status, st);
   if (D == 256) return launch_fwd<256>(q, k, v, out, lse, B, Sq, Skv, Hq, Hkv, scale, causal, q_pos0, k_pos0, status, st);

@@ -714,15 +714,10 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// 2-D bf16 tensor map with 128-byte swizzle. `inner` is the contiguous extent.
-static int encode_tensor_map_2d_impl(CUtensorMap* out, const void* base, int elem_bytes, uint64_t inner,
-                                     uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner,
-                                     uint32_t box_outer);
-static inline int encode_tensor_map_2d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t inner,
-                                       uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner,
-                                       uint32_t box_outer) {
-  return encode_tensor_map_2d_impl(out, base, elem_bytes, inner, outer, row_stride_bytes, box_inner, box_outer);
-}
+// Tensor map with 128-byte swizzle over [outer, inner] rows, or over [depth, outer, inner] with depth > 0.
+static int encode_tensor_map(CUtensorMap* out, const void* base, int elem_bytes, uint64_t inner, uint64_t outer,
+                             uint64_t depth, uint64_t row_stride_bytes, uint64_t depth_stride_bytes, uint32_t box_inner,
+                             uint32_t box_outer);
 
 // A tensor map is a pure function of (base, element size, extents, row stride, box): training re-issues the same
 // few hundred (pointer, shape) pairs every step - weights, the flat gradient, cached activation buffers - so the
@@ -731,11 +726,12 @@ static inline int encode_tensor_map_2d(CUtensorMap* out, const void* base, int e
 namespace {
 struct MapKey {
   const void* base;
-  uint64_t inner, outer, stride;
+  uint64_t inner, outer, depth, stride, depth_stride;
   uint32_t box_inner, box_outer;
   int elem;
   bool operator==(const MapKey& o) const {
-    return base == o.base && inner == o.inner && outer == o.outer && stride == o.stride &&
+    return base == o.base && inner == o.inner && outer == o.outer && depth == o.depth && stride == o.stride &&
+           depth_stride == o.depth_stride &&
            box_inner == o.box_inner && box_outer == o.box_outer && elem == o.elem;
   }
 };
@@ -749,7 +745,7 @@ inline uint64_t map_hash(const MapKey& k) {
   uint64_t h = reinterpret_cast<uint64_t>(k.base) * 0x9E3779B97F4A7C15ull;
   h ^= (k.inner + 0x632BE59BD9B4E019ull) * 0xC2B2AE3D27D4EB4Full;
   h ^= (k.outer << 20) ^ (k.stride << 7) ^ (static_cast<uint64_t>(k.box_inner) << 40) ^
-       (static_cast<uint64_t>(k.box_outer) << 52) ^ static_cast<uint64_t>(k.elem);
+       (static_cast<uint64_t>(k.box_outer) << 52) ^ static_cast<uint64_t>(k.elem) ^ (k.depth * 0xD6E8FEB86659FD93ull);
   h ^= h >> 29;
   return h * 0xBF58476D1CE4E5B9ull;
 }
@@ -757,9 +753,15 @@ inline uint64_t map_hash(const MapKey& k) {
 
 int make_tensor_map_2d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t inner, uint64_t outer,
                        uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer) {
+  return make_tensor_map_3d(out, base, elem_bytes, inner, outer, 0, row_stride_bytes, 0, box_inner, box_outer);
+}
+
+int make_tensor_map_3d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t inner, uint64_t outer,
+                       uint64_t depth, uint64_t row_stride_bytes, uint64_t depth_stride_bytes, uint32_t box_inner,
+                       uint32_t box_outer) {
   static const bool cache_on = [] { const char* e = getenv("CVERL_B200_TMAP_CACHE"); return !(e && e[0] == '0'); }();
   static thread_local MapSlot* table = nullptr;
-  const MapKey key{base, inner, outer, row_stride_bytes, box_inner, box_outer, elem_bytes};
+  const MapKey key{base, inner, outer, depth, row_stride_bytes, depth_stride_bytes, box_inner, box_outer, elem_bytes};
   MapSlot* slot = nullptr;
   if (cache_on) {
     if (!table) table = static_cast<MapSlot*>(calloc(MAP_CACHE_SLOTS, sizeof(MapSlot)));
@@ -778,7 +780,8 @@ int make_tensor_map_2d(CUtensorMap* out, const void* base, int elem_bytes, uint6
       if (!slot) slot = &table[map_hash(key) & (MAP_CACHE_SLOTS - 1)];  // full neighbourhood: overwrite
     }
   }
-  const int rc = encode_tensor_map_2d(out, base, elem_bytes, inner, outer, row_stride_bytes, box_inner, box_outer);
+  const int rc = encode_tensor_map(out, base, elem_bytes, inner, outer, depth, row_stride_bytes, depth_stride_bytes,
+                                   box_inner, box_outer);
   if (rc == 0 && slot) {
     slot->key = key;
     slot->map = *out;
@@ -787,9 +790,9 @@ int make_tensor_map_2d(CUtensorMap* out, const void* base, int elem_bytes, uint6
   return rc;
 }
 
-static int encode_tensor_map_2d_impl(CUtensorMap* out, const void* base, int elem_bytes, uint64_t inner,
-                                     uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner,
-                                     uint32_t box_outer) {
+static int encode_tensor_map(CUtensorMap* out, const void* base, int elem_bytes, uint64_t inner, uint64_t outer,
+                             uint64_t depth, uint64_t row_stride_bytes, uint64_t depth_stride_bytes, uint32_t box_inner,
+                             uint32_t box_outer) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return -1;
   // The driver call needs this thread to have a current context.  Autograd runs backward on
@@ -799,12 +802,12 @@ static int encode_tensor_map_2d_impl(CUtensorMap* out, const void* base, int ele
     cudaFree(nullptr);
     context_bound = true;
   }
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {row_stride_bytes};
-  cuuint32_t box[2] = {box_inner, box_outer};
-  cuuint32_t estr[2] = {1, 1};
+  cuuint64_t dims[3] = {inner, outer, depth};
+  cuuint64_t strides[2] = {row_stride_bytes, depth_stride_bytes};
+  cuuint32_t box[3] = {box_inner, box_outer, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
   CUtensorMapDataType dt = elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  CUresult r = fn(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  CUresult r = fn(out, dt, depth > 0 ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {

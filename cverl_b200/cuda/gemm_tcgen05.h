@@ -101,5 +101,9 @@ struct GemmParams {
 };
 int make_tensor_map_2d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t inner, uint64_t outer,
                        uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer);
+// [depth, outer, inner]: a box of one depth index never reaches into the next, rows past `outer` read as zero
+int make_tensor_map_3d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t inner, uint64_t outer,
+                       uint64_t depth, uint64_t row_stride_bytes, uint64_t depth_stride_bytes, uint32_t box_inner,
+                       uint32_t box_outer);
 }  // namespace cvb
 #endif
