@@ -107,7 +107,7 @@ _CUDA_PROTOS = {
     "cvb_p2p_scatter_rows": "pp i pp ll l p p",
     "cvb_p2p_gather_rows": "pp i pp ll l p p",
     "cvb_attention_fwd": "ppppp l iiiii f i ll p p",
-    "cvb_attention_bwd": "ppppp p pp ppp l iiiii f i ll p p",
+    "cvb_attention_bwd": "ppppp p p ppp l iiiii f i ll p p",
     "cvb_attn_merge": "pppp l iiiiii p",
     "cvb_decode_attention": "p ll pp l ppp p iiiii f p p",
     "cvb_gdn_decode_step": "p l ii pp i p pp l pp pp i p",

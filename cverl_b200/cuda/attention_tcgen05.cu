@@ -26,6 +26,7 @@
 #include "ptx.cuh"
 #include "gemm_tcgen05.h"
 #include <initializer_list>
+#include <type_traits>
 
 namespace cvb {
 
@@ -414,7 +415,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int c = 0; c < NB; ++c)
           tma_store_3d(&tmO, stage + c * 16384, h * D + c * 64, q0 + t * AT_BQ, b);
         tma_store_commit();
-        tma_store_wait_all();
+        tma_store_wait_read();
       }
     }
   }
@@ -480,52 +481,64 @@ extern "C" int cvb_attention_fwd(const void* q, const void* k, const void* v, vo
 // =================================================================================================
 // Backward.
 //
-// One CTA per (128-key block, query head, batch) walks the query blocks (64 queries) that can see it.
-// Everything is computed transposed, keys on the TMEM lanes, so that each thread owns one key row:
-//     S^T  = K Q^T          dP^T = V dO^T                    (M = 128 keys, N = 64 queries, K = D)
-//     P^T  = exp2(S^T c - LSE_q)        dS^T = P^T (dP^T - Delta_q) * scale
-//     dV  += P^T dO         dK  += dS^T Q                    (N = D, K = 64; dO / Q read MN-major)
-//     dQ^T = K^T dS^T                                        (M = D in chunks of 128, N = 64, K = 128 keys)
-// dV and dK stay in TMEM for the whole CTA; dQ^T of each (key block, query block) pair is added to a
-// transposed fp32 buffer [B, Hq, D, Sq] with 16-byte vector reductions (a thread holds 64 consecutive
-// queries of one d), and a last kernel turns that buffer into bf16 [B, Sq, Hq, D].
-// TMEM has 512 columns: with D = 128 everything fits in one kernel (MODE 0); with D = 256 the work is
-// split into a dV kernel (MODE 1: S^T, dV) and a dK / dQ kernel (MODE 2: S^T, dP^T, dK, dQ^T).
-// A CTA walks the query blocks of EVERY query head of its GQA group, so dK / dV come out already summed.
+// One kernel template in four roles, each with an accumulator that stays in TMEM for the whole CTA:
+//   BWD_Q   rows = 128 queries, walks the keys:     dQ += dS K
+//   BWD_K   rows = 128 keys, walks the queries:     dK += dS^T Q                    (head dim 256)
+//   BWD_V   rows = 128 keys, walks the queries:     dV += P^T dO                    (head dim 256)
+//   BWD_KV  both of the last two in one CTA                                         (head dim 128)
+// At head dim 256 the accumulators of dK and dV alone fill the 512 TMEM columns, so the two are separate launches.
+// The walk goes in steps of 64 columns (queries or keys).  With A1, A2 the CTA's own rows (K and V, or Q and dO) and
+// B1, B2 the step's rows of the other side (Q and dO, or K and V):
+//     S  = A1 B1^T       dP = A2 B2^T           M = 128, N = 64, K = D
+//     P  = exp2(S c - LSE)          dS = P (dP - Delta) scale
+//     acc += dS B1  (and acc_v += P B2)         M = 128, N = D, K = 64, B read MN-major
+// dQ needs no reduction across CTAs (no zeroed fp32 buffer, no transposing pass over it) at the price of forming S and
+// dP once more.
+// What makes the pipeline fit into 227 KB at head dim 256: A2 is copied once into 128 TMEM columns and read from there
+// as the A operand, which leaves three slots for the operand that is held until its accumulate step and one for the
+// other; S and dP have one TMEM buffer each, which the softmax warps empty into registers and release at once.  The
+// tensor cores then run S, dP of step j + 1 while the warps form dS of step j, and the accumulate step of j while
+// the warps fetch S, dP of j + 1.
+// Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 two warpgroups that split the 64 columns of a step.
+// A CTA of BWD_K / BWD_V / BWD_KV walks the queries of EVERY head of its GQA group, so dK / dV come out summed.
+// Causal, 16 x 1280 with 8 query and 2 kv heads of 256: dQ 230, dK 207, dV 143 and Delta 37 us; one serial chain of MMA
+// and softmax per CTA in two kernels, with dQ reduced into a cleared fp32 buffer and transposed, took 1,130.  A step of
+// 64 columns of BWD_K takes about 1.9 us: three MMA units against 64 KB of operands, as many bytes per unit as the
+// forward reads.
 // =================================================================================================
-constexpr int AB_BKV = 128;  // keys per CTA
-constexpr int AB_BQ = 64;    // queries per step
-// Two warpgroups: warps w and w + 4 share TMEM lane quadrant w (the same 32 keys) and split the 32-column chunks
-// of every TMEM -> registers hand-off between the two MMA rounds of a step.
-constexpr int AB_THREADS = 256;
+constexpr int AB_ROWS = 128;   // rows per CTA
+constexpr int AB_STEP = 64;    // columns per step
+constexpr int AB_THREADS = 320;
+
+enum : int { BWD_Q = 0, BWD_K = 1, BWD_V = 2, BWD_KV = 3 };
 
 template <int D, int MODE>
 struct AttBwdCfg {
-  static constexpr bool NEED_V = MODE != 1;
-  static constexpr bool NEED_PT = MODE != 2;
-  static constexpr bool NEED_DS = MODE != 1;
-  static constexpr int NBUF = (MODE == 2 && D == 256) ? 1 : 2;
-  static constexpr int K = 0;                                   // D/64 boxes [128 x 64]
-  static constexpr int V = K + D * 256;
-  static constexpr int Q = V + (NEED_V ? D * 256 : 0);          // NBUF x D/64 boxes [64 x 64]
-  static constexpr int DO = Q + NBUF * D * 128;
-  static constexpr int PT = DO + NBUF * D * 128;                // [128 x 64] bf16
-  static constexpr int DS = PT + (NEED_PT ? 16384 : 0);
-  static constexpr int VEC = DS + (NEED_DS ? 16384 : 0);        // lse2[NBUF][64], delta[NBUF][64]
-  static constexpr int BARS = VEC + 1024;
+  static constexpr bool ROWQ = MODE == BWD_Q;              // rows are queries
+  static constexpr bool HAS_DP = MODE != BWD_V;
+  static constexpr bool ACC_1 = MODE != BWD_V;             // acc += dS B1
+  static constexpr bool ACC_V = MODE == BWD_V || MODE == BWD_KV;
+  static constexpr int BLOCK = D * 128;                    // bytes of one [64 x D] block
+  // ring 1 holds B1, ring 2 holds B2.  An operand that an accumulate step reads is held for a whole step longer than
+  // one that only S or dP reads; BWD_V takes them in different MMAs and balances the two.
+  static constexpr int N1 = MODE == BWD_V ? 2 : 3;
+  static constexpr int N2 = MODE == BWD_V ? 2 : (MODE == BWD_KV ? 3 : (D == 128 ? 2 : 1));
+  static constexpr int A1 = 0;                             // D/64 boxes [128 x 64]
+  static constexpr int R1 = A1 + D * 256;
+  static constexpr int R2 = R1 + N1 * BLOCK;
+  static constexpr int PT = R2 + N2 * BLOCK;               // P   [128 x 64] bf16
+  static constexpr int DS = PT + (ACC_V ? 16384 : 0);      // dS  [128 x 64] bf16
+  static constexpr int VEC = DS + (ACC_1 ? 16384 : 0);     // per warp: lse2[32], delta[32]
+  static constexpr int BARS = VEC + 2048;
   static constexpr int BYTES = BARS + 256 + 1024;
-  static constexpr uint32_t TC_S = 0, TC_DP = 64;
-  static constexpr uint32_t TC_DV = (MODE == 1) ? 64 : 128;
-  static constexpr uint32_t TC_DK = (MODE == 0) ? 128 + D : 128;
-  static constexpr uint32_t TC_DQ = 384;
+  static constexpr int STG_A2 = R1 + BLOCK;                // A2 on its way to TMEM: slots 1 and 2 of ring 1
+  static constexpr int STG_V = (MODE == BWD_KV) ? R2 : A1; // dV on its way out
+  static constexpr uint32_t TC_1 = 0, TC_V = (MODE == BWD_KV) ? D : 0, TC_A2 = 256, TC_S = 384, TC_DP = 448;
 };
 
 struct AttBwdArgs {
   const float* lse;      // [B, Hq, Sq] natural log
   const float* delta;    // [B, Hq, Sq] rowsum(dO * O)
-  __nv_bfloat16* dk;     // [B, Skv, Hkv, D]
-  __nv_bfloat16* dv;     // [B, Skv, Hkv, D]
-  float* dqt;            // [B, Hq, D, Sq] fp32, zero-initialised, accumulated with reductions
   int Sq, Skv, Hq, Hkv, B;
   float scale, scale_log2;
   int causal;
@@ -533,77 +546,84 @@ struct AttBwdArgs {
   int* status;
 };
 
+// Maps: tmA1 / tmA2 boxes of 128 rows, tmB1 / tmB2 boxes of 64 rows, tmO1 (dQ or dK) / tmOV (dV) boxes of 128 rows.
 template <int D, int MODE>
 __global__ void __launch_bounds__(AB_THREADS, 1)
-attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
+attention_bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmA2,
+                     const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmB2,
+                     const __grid_constant__ CUtensorMap tmO1, const __grid_constant__ CUtensorMap tmOV,
                      const AttBwdArgs a) {
   using C = AttBwdCfg<D, MODE>;
   constexpr int NB = D / 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::BARS);
-  uint64_t *bar_kv = bars, *bar_q = bars + 1 /* [2] */, *bar_1 = bars + 3, *bar_2 = bars + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* bar_a = bars;            // A1 has landed
+  uint64_t* bar_a2 = bars + 1;       // A2 is in TMEM
+  uint64_t* bar_sd = bars + 2;       // S and dP of a step are complete
+  uint64_t* bar_free = bars + 3;     // S and dP have been read
+  uint64_t* bar_ds = bars + 4;       // P / dS of a step are in shared memory
+  uint64_t* bar_acc = bars + 5;      // the accumulate step is complete
+  uint64_t* full1 = bars + 6;        // [3]
+  uint64_t* empty1 = bars + 9;       // [3]
+  uint64_t* full2 = bars + 12;       // [3]
+  uint64_t* empty2 = bars + 15;      // [3]
+  uint64_t* bar_out = bars + 18;     // the result is staged
+  uint64_t* bar_a2s = bars + 19;     // A2 has landed in its staging slots
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* s_lse2 = reinterpret_cast<float*>(smem + C::VEC);         // [NBUF][64]
-  float* s_delta = s_lse2 + 2 * AB_BQ;
 
-  const int tid = threadIdx.x;
-  const int wg = tid >> 7;      // warpgroup: every second 32-column chunk
-  const int lt = tid & 127;     // key row of this thread = its TMEM lane
-  const int warp = lt >> 5;     // TMEM lane quadrant
-  // 1-D grid with the key block slowest: causal key blocks near the start see the most queries, so the
-  // longest CTAs are scheduled first and the tail of the launch consists of short ones.
-  const int per_block = a.Hkv * a.B;                        // (kv head, batch) pairs per key block
-  const int k0 = (blockIdx.x / per_block) * AB_BKV;
-  const int hk = (blockIdx.x % per_block) % a.Hkv;
-  const long long b = (blockIdx.x % per_block) / a.Hkv;
-  const int group = a.Hq / a.Hkv;                           // query heads that share this kv head
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sb = smem_u32(smem);
-  const long long kpos = a.k_pos0 + k0 + lt;
+  const int group = a.Hq / a.Hkv;   // query heads that share a kv head
+  // 1-D grid, row block slowest and the longest first: under the causal mask late queries see the most keys and
+  // early keys are seen by the most queries.
+  const int heads = C::ROWQ ? a.Hq : a.Hkv;
+  const int per_block = heads * a.B;
+  const int row_blocks = ((C::ROWQ ? a.Sq : a.Skv) + AB_ROWS - 1) / AB_ROWS;
+  const int blk = static_cast<int>(blockIdx.x) / per_block;
+  const int r0 = (C::ROWQ ? row_blocks - 1 - blk : blk) * AB_ROWS;
+  const int head = static_cast<int>(blockIdx.x % per_block) % heads;
+  const int b = static_cast<int>(blockIdx.x % per_block) / heads;
+  const int hq0 = C::ROWQ ? head : head * group;
+  const int hk = C::ROWQ ? head / group : head;
 
-  const int nq = a.Sq / AB_BQ;
-  int m_begin = 0;
-  if (a.causal) {   // first query block with a query at or after this block's first key
-    const long long need = a.k_pos0 + k0 - a.q_pos0 - (AB_BQ - 1);
-    m_begin = need <= 0 ? 0 : static_cast<int>((need + AB_BQ - 1) / AB_BQ);
-    if (m_begin > nq) m_begin = nq;
-  }
-  const int per_head = nq - m_begin;          // query blocks per head that see this key block
-  const int steps = per_head * group;         // dK / dV accumulate over every query head of the GQA group
-
-  auto load_q = [&](int it) {
-    const int buf = it % C::NBUF;
-    const int m = m_begin + it % per_head;
-    const int h = hk * group + it / per_head;
-    const int qrow = static_cast<int>(b * a.Sq + static_cast<long long>(m) * AB_BQ);
-    mbar_arrive_expect_tx(&bar_q[buf], 2u * D * 128u);
-#pragma unroll
-    for (int c = 0; c < NB; ++c) {
-      tma_load_2d(smem + C::Q + buf * (D * 128) + c * 8192, &tmQ, &bar_q[buf], h * D + c * 64, qrow);
-      tma_load_2d(smem + C::DO + buf * (D * 128) + c * 8192, &tmDO, &bar_q[buf], h * D + c * 64, qrow);
+  // steps: column blocks [c_begin, c_end) for each query head of the group
+  int c_begin = 0, c_end = ((C::ROWQ ? a.Skv : a.Sq) + AB_STEP - 1) / AB_STEP;
+  if (a.causal) {
+    if (C::ROWQ) {   // keys up to the last query of the block
+      const long long lim = a.q_pos0 + min(r0 + AB_ROWS, a.Sq) - 1 - a.k_pos0;
+      c_end = lim < 0 ? 0 : static_cast<int>(min(static_cast<long long>(c_end), lim / AB_STEP + 1));
+    } else {         // queries from the first key of the block on
+      const long long need = a.k_pos0 + r0 - a.q_pos0 - (AB_STEP - 1);
+      if (need > 0) c_begin = static_cast<int>(min(static_cast<long long>(c_end), (need + AB_STEP - 1) / AB_STEP));
     }
-  };
+  }
+  const int per_head = c_end - c_begin;
+  const int steps = per_head * (C::ROWQ ? 1 : group);
 
   if (tid == 0) {
-    mbar_init(bar_kv, 1); mbar_init(&bar_q[0], 1); mbar_init(&bar_q[1], 1); mbar_init(bar_1, 1); mbar_init(bar_2, 1);
+    mbar_init(bar_a, 1);
+    mbar_init(bar_a2, 8);
+    mbar_init(bar_a2s, 1);
+    mbar_init(bar_sd, 1);
+    mbar_init(bar_free, 8);
+    mbar_init(bar_ds, 8);
+    mbar_init(bar_acc, 1);
+    mbar_init(bar_out, 8);
+    for (int s = 0; s < 3; ++s) {
+      mbar_init(&full1[s], 1);
+      mbar_init(&empty1[s], 1);
+      mbar_init(&full2[s], 1);
+      mbar_init(&empty2[s], 1);
+    }
     *abort_flag = 0;
     mbar_fence_init();
-    if (steps > 0) {
-      mbar_arrive_expect_tx(bar_kv, (C::NEED_V ? 2u : 1u) * D * 256u);
-      const int krow = static_cast<int>(b * a.Skv + k0);
-#pragma unroll
-      for (int c = 0; c < NB; ++c) {
-        tma_load_2d(smem + C::K + c * 16384, &tmK, bar_kv, hk * D + c * 64, krow);
-        if (C::NEED_V) tma_load_2d(smem + C::V + c * 16384, &tmV, bar_kv, hk * D + c * 64, krow);
-      }
-      load_q(0);
-      if (C::NBUF == 2 && steps > 1) load_q(1);
-    }
+    tma_prefetch_desc(&tmA1);
+    tma_prefetch_desc(&tmB1);
+    tma_prefetch_desc(&tmB2);
   }
-  if (tid < 32) {
-    __syncwarp();
+  if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
@@ -611,201 +631,301 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
 
-  bool ok = true;
-  if (steps > 0) {
-    if (!mbar_wait_bounded(bar_kv, 0, abort_flag)) {
-      if (!*abort_flag) atomicCAS(a.status, 0, ERR_WAIT_FULL);
-      *abort_flag = 1;
+  auto fail = [&](int code) {
+    if (!*abort_flag) atomicCAS(a.status, 0, code);
+    *abort_flag = 1;
+  };
+
+  if (warp == 0) {
+    // ------------------------------ TMA producer ------------------------------
+    if (lane == 0 && steps > 0) {
+      const int ha = C::ROWQ ? head : hk;
+      mbar_arrive_expect_tx(bar_a, D * 256u);
+#pragma unroll
+      for (int c = 0; c < NB; ++c) tma_load_3d(smem + C::A1 + c * 16384, &tmA1, bar_a, ha * D + c * 64, r0, b);
+      bool ok = true;
+      uint32_t armed = 0, parity = 0;
+      // slot and phase of step j in a ring of n slots
+      auto load = [&](int j, int ring) {
+        const int n = ring == 1 ? C::N1 : C::N2;
+        const int slot = j % n;
+        const uint32_t ph = (j / n) & 1;
+        uint64_t* fb = (ring == 1 ? full1 : full2) + slot;
+        if (!mbar_wait_bounded((ring == 1 ? empty1 : empty2) + slot, ph ^ 1, abort_flag)) {
+          fail(ERR_WAIT_EMPTY);
+          ok = false;
+          return;
+        }
+        const int col = (c_begin + j % per_head) * AB_STEP;
+        const int hb = C::ROWQ ? hk : hq0 + j / per_head;
+        uint8_t* dst = smem + (ring == 1 ? C::R1 : C::R2) + slot * C::BLOCK;
+        mbar_arrive_expect_tx(fb, C::BLOCK);
+#pragma unroll
+        for (int c = 0; c < NB; ++c)
+          tma_load_3d(dst + c * 8192, ring == 1 ? &tmB1 : &tmB2, fb, hb * D + c * 64, col, b);
+        const int bit = (ring == 1 ? 0 : 3) + slot;
+        armed |= 1u << bit;
+        parity = (parity & ~(1u << bit)) | (ph << bit);
+      };
+      load(0, 1);     // S of step 0 starts while A2 is on its way
+      if (C::HAS_DP) {
+        mbar_arrive_expect_tx(bar_a2s, D * 256u);
+#pragma unroll
+        for (int c = 0; c < NB; ++c) tma_load_3d(smem + C::STG_A2 + c * 16384, &tmA2, bar_a2s, ha * D + c * 64, r0, b);
+      }
+      if (ok) load(0, 2);
+      if (ok && C::HAS_DP && !mbar_wait_bounded(bar_a2, 0, abort_flag)) {   // slots 1 and 2 of ring 1 held A2
+        fail(ERR_WAIT_EMPTY);
+        ok = false;
+      }
+      for (int j = 1; j < steps && ok; ++j) {
+        load(j, 1);
+        if (ok) load(j, 2);
+      }
+      if (!ok || *abort_flag) {   // leave no copy in flight
+        int dummy = 0;
+        mbar_wait_bounded(bar_a, 0, &dummy);
+        if (C::HAS_DP) mbar_wait_bounded(bar_a2s, 0, &dummy);
+        for (int s = 0; s < 6; ++s)
+          if (armed & (1u << s)) mbar_wait_bounded((s < 3 ? full1 + s : full2 + s - 3), (parity >> s) & 1, &dummy);
+      }
     }
-    __syncthreads();
-    ok = !*abort_flag;
-  }
-  for (int it = 0; it < steps && ok; ++it) {
-    const int buf = it % C::NBUF;
-    const int m = m_begin + it % per_head;
-    const int h = hk * group + it / per_head;
-    const uint32_t phq = (it / C::NBUF) & 1, pit = it & 1;
-    const uint32_t qb = sb + C::Q + buf * (D * 128), dob = sb + C::DO + buf * (D * 128);
-    // per-query scalars of this block
-    if (tid < AB_BQ) {
-      const long long qi = (b * a.Hq + h) * a.Sq + static_cast<long long>(m) * AB_BQ + tid;
-      s_lse2[buf * AB_BQ + tid] = a.lse[qi] * 1.4426950408889634f;
-      s_delta[buf * AB_BQ + tid] = a.delta[qi];
-    }
-    // ---- MMA phase 1: S^T = K Q^T (and dP^T = V dO^T) ---------------------------------------------------------
-    if (tid == 0) {
-      if (mbar_wait_bounded(&bar_q[buf], phq, abort_flag)) {
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer --------------------------------
+    if (lane == 0 && steps > 0) {
+      constexpr uint32_t id_s = umma_idesc(128, AB_STEP, 1, 0, 0);
+      constexpr uint32_t id_acc = umma_idesc(128, D, 1, 0, 1);
+      bool ok = true;
+      auto wait = [&](uint64_t* bar, uint32_t par, int code) {
+        if (ok && !mbar_wait_bounded(bar, par, abort_flag)) {
+          fail(code);
+          ok = false;
+        }
+      };
+      auto scores = [&](int j) {   // S (and dP) of step j
+        const int s1 = j % C::N1, s2 = j % C::N2;
+        wait(&full1[s1], (j / C::N1) & 1, ERR_WAIT_FULL);
+        if (!ok) return;
         tc_fence_after();
-        constexpr uint32_t idesc = umma_idesc(128, AB_BQ, 1, 0, 0);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t kb = k >> 2, ks = (k & 3) * 32;
-          umma_bf16(tmem_base + C::TC_S, umma_smem_desc(sb + C::K + kb * 16384 + ks, 16, 1024),
-                    umma_smem_desc(qb + kb * 8192 + ks, 16, 1024), idesc, k > 0);
+          umma_bf16(tmem_base + C::TC_S, umma_smem_desc(sb + C::A1 + kb * 16384 + ks, 16, 1024),
+                    umma_smem_desc(sb + C::R1 + s1 * C::BLOCK + kb * 8192 + ks, 16, 1024), id_s, k > 0);
         }
-        if (C::NEED_DS) {
+        if (!C::ACC_1) umma_commit(&empty1[s1]);
+        if (C::HAS_DP) {
+          if (j == 0) wait(bar_a2, 0, ERR_WAIT_FULL);
+          wait(&full2[s2], (j / C::N2) & 1, ERR_WAIT_FULL);
+          if (!ok) return;
+          tc_fence_after();
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) {
             const uint32_t kb = k >> 2, ks = (k & 3) * 32;
-            umma_bf16(tmem_base + C::TC_DP, umma_smem_desc(sb + C::V + kb * 16384 + ks, 16, 1024),
-                      umma_smem_desc(dob + kb * 8192 + ks, 16, 1024), idesc, k > 0);
+            umma_bf16_ts(tmem_base + C::TC_DP, tmem_base + C::TC_A2 + k * 8,
+                         umma_smem_desc(sb + C::R2 + s2 * C::BLOCK + kb * 8192 + ks, 16, 1024), id_s, k > 0);
           }
+          if (!C::ACC_V) umma_commit(&empty2[s2]);
         }
-        umma_commit(bar_1);
-      } else {
-        if (!*abort_flag) atomicCAS(a.status, 0, ERR_WAIT_FULL);
-        *abort_flag = 1;
+        umma_commit(bar_sd);
+      };
+      wait(bar_a, 0, ERR_WAIT_FULL);
+      if (ok) scores(0);
+      for (int j = 0; j < steps && ok; ++j) {
+        if (j + 1 < steps) {
+          wait(bar_free, j & 1, ERR_WAIT_TMEM_EMPTY);
+          if (!ok) break;
+          scores(j + 1);
+          if (!ok) break;
+        }
+        const int s1 = j % C::N1, s2 = j % C::N2;
+        wait(bar_ds, j & 1, ERR_WAIT_TMEM_EMPTY);
+        if (C::ACC_V && !C::HAS_DP) wait(&full2[s2], (j / C::N2) & 1, ERR_WAIT_FULL);
+        if (!ok) break;
+        tc_fence_after();
+        if (C::ACC_V) {
+#pragma unroll
+          for (int k = 0; k < AB_STEP / 16; ++k)
+            umma_bf16(tmem_base + C::TC_V, umma_smem_desc(sb + C::PT + k * 32, 16, 1024),
+                      umma_smem_desc(sb + C::R2 + s2 * C::BLOCK + k * 2048, 8192, 1024), id_acc, (j > 0 || k > 0));
+          umma_commit(&empty2[s2]);
+        }
+        if (C::ACC_1) {
+#pragma unroll
+          for (int k = 0; k < AB_STEP / 16; ++k)
+            umma_bf16(tmem_base + C::TC_1, umma_smem_desc(sb + C::DS + k * 32, 16, 1024),
+                      umma_smem_desc(sb + C::R1 + s1 * C::BLOCK + k * 2048, 8192, 1024), id_acc, (j > 0 || k > 0));
+          umma_commit(&empty1[s1]);
+        }
+        umma_commit(bar_acc);
       }
     }
-    if (!mbar_wait_bounded(bar_1, pit, abort_flag)) {
-      if (!*abort_flag) atomicCAS(a.status, 0, ERR_WAIT_TMEM_FULL);
-      *abort_flag = 1;
+  } else {
+    // ------------------------------ P and dS, one row per thread and half ---------------
+    const int wg = warp >= 6 ? 1 : 0;       // columns [32 wg, 32 wg + 32) of every step
+    const int quad = warp & 3;              // TMEM lane quadrant of this warp
+    const int row = quad * 32 + lane;
+    float* v_lse2 = reinterpret_cast<float*>(smem + C::VEC) + (warp - 2) * 64;
+    float* v_delta = v_lse2 + 32;
+    const uint32_t tmem = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+    const int ri = r0 + row;
+    bool ok = true;
+    auto wait = [&](uint64_t* bar, uint32_t par) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, par, abort_flag));
+      if (!ok && lane == 0) fail(ERR_WAIT_TMEM_FULL);
+      return ok;
+    };
+    // queries past the end, and queries that see no key, get LSE = +inf: their P is exp2(-inf) = 0
+    auto lse2_of = [](float lse) { return lse > -INFINITY ? lse * 1.4426950408889634f : INFINITY; };
+    float row_lse2 = INFINITY, row_delta = 0.f;
+    if (C::ROWQ && ri < a.Sq) {
+      const long long i = (static_cast<long long>(b) * a.Hq + head) * a.Sq + ri;
+      row_lse2 = lse2_of(a.lse[i]);
+      row_delta = a.delta[i];
     }
-    __syncthreads();   // also publishes s_lse2 / s_delta
-    if (*abort_flag) { ok = false; break; }
-    tc_fence_after();
-    // ---- P^T and dS^T rows (one key per thread) ------------------------------------------------------------
-    {
-      const long long qbase = a.q_pos0 + static_cast<long long>(m) * AB_BQ;
-      const bool diag = a.causal && (kpos > qbase);      // some query of the block is before this key
-      // queries [first_vis, 64) see this key
-      int first_vis = 0;
-      if (diag) {
-        const long long f = kpos - qbase;
-        first_vis = f > AB_BQ ? AB_BQ : static_cast<int>(f);
-      }
+    if (C::HAS_DP && steps > 0 && wait(bar_a2s, 0)) {
+      // this row's A2 into TMEM, two bf16 per column: the A operand of dP
 #pragma unroll 1
-      for (int c0 = wg * 32; c0 < AB_BQ; c0 += 64) {
-        uint32_t rs[32], rp[32];
-        tmem_ld_32x32(tmem + C::TC_S + c0, rs);
-        if (C::NEED_DS) tmem_ld_32x32(tmem + C::TC_DP + c0, rp);
-        tmem_ld_wait();
-        float p[32], ds[32];
+      for (int c = wg * (NB / 2); c < (wg + 1) * (NB / 2); ++c) {
+        uint32_t r[32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int qi = c0 + i;
-          const float l2 = s_lse2[buf * AB_BQ + qi];
-          const bool vis = qi >= first_vis && l2 > -INFINITY;
-          p[i] = vis ? exp2f(__uint_as_float(rs[i]) * a.scale_log2 - l2) : 0.f;
-          if (C::NEED_DS) ds[i] = p[i] * (__uint_as_float(rp[i]) - s_delta[buf * AB_BQ + qi]) * a.scale;
+        for (int i = 0; i < 8; ++i) {
+          const uint4 u = *reinterpret_cast<const uint4*>(smem + C::STG_A2 + c * 16384 + asw128(row, i));
+          r[4 * i] = u.x;
+          r[4 * i + 1] = u.y;
+          r[4 * i + 2] = u.z;
+          r[4 * i + 3] = u.w;
         }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint32_t off = asw128(lt, (c0 >> 3) + c);
-          if (C::NEED_PT) {
-            uint4 u;
-            u.x = pack_bf16x2(p[8 * c + 0], p[8 * c + 1]); u.y = pack_bf16x2(p[8 * c + 2], p[8 * c + 3]);
-            u.z = pack_bf16x2(p[8 * c + 4], p[8 * c + 5]); u.w = pack_bf16x2(p[8 * c + 6], p[8 * c + 7]);
-            *reinterpret_cast<uint4*>(smem + C::PT + off) = u;
-          }
-          if (C::NEED_DS) {
-            uint4 u;
-            u.x = pack_bf16x2(ds[8 * c + 0], ds[8 * c + 1]); u.y = pack_bf16x2(ds[8 * c + 2], ds[8 * c + 3]);
-            u.z = pack_bf16x2(ds[8 * c + 4], ds[8 * c + 5]); u.w = pack_bf16x2(ds[8 * c + 6], ds[8 * c + 7]);
-            *reinterpret_cast<uint4*>(smem + C::DS + off) = u;
-          }
-        }
+        tmem_st_32x32(tmem + C::TC_A2 + c * 32, r);
       }
-    }
-    fence_proxy_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    // ---- MMA phase 2: dV += P^T dO, dK += dS^T Q, dQ^T = K^T dS^T -------------------------------------------
-    if (tid == 0) {
-      constexpr uint32_t id_acc = umma_idesc(128, D, 1, 0, 1);
-      if (C::NEED_PT) {
-#pragma unroll
-        for (int k = 0; k < AB_BQ / 16; ++k)
-          umma_bf16(tmem_base + C::TC_DV, umma_smem_desc(sb + C::PT + k * 32, 16, 1024),
-                    umma_smem_desc(dob + k * 2048, 8192, 1024), id_acc, (it > 0 || k > 0));
-      }
-      if (C::NEED_DS) {
-#pragma unroll
-        for (int k = 0; k < AB_BQ / 16; ++k)
-          umma_bf16(tmem_base + C::TC_DK, umma_smem_desc(sb + C::DS + k * 32, 16, 1024),
-                    umma_smem_desc(qb + k * 2048, 8192, 1024), id_acc, (it > 0 || k > 0));
-        constexpr uint32_t id_dq = umma_idesc(128, AB_BQ, 1, 1, 1);
-#pragma unroll
-        for (int ch = 0; ch < D / 128; ++ch) {
-#pragma unroll
-          for (int k = 0; k < AB_BKV / 16; ++k)
-            umma_bf16(tmem_base + C::TC_DQ + ch * AB_BQ,
-                      umma_smem_desc(sb + C::K + ch * 32768 + k * 2048, 16384, 1024),
-                      umma_smem_desc(sb + C::DS + k * 2048, 16, 1024), id_dq, k > 0);
-        }
-      }
-      umma_commit(bar_2);
-    }
-    if (!mbar_wait_bounded(bar_2, pit, abort_flag)) {
-      if (!*abort_flag) atomicCAS(a.status, 0, ERR_WAIT_TMEM_FULL);
-      *abort_flag = 1;
-    }
-    __syncthreads();
-    if (*abort_flag) { ok = false; break; }
-    tc_fence_after();
-    if (tid == 0 && it + C::NBUF < steps) load_q(it + C::NBUF);   // Q / dO buffer is free again
-    if (C::NEED_DS) {
-      // dQ^T chunk rows: lane = d, 64 consecutive queries -> vector reductions into [B, Hq, D, Sq]
-#pragma unroll 1
-      for (int ch = 0; ch < D / 128; ++ch) {
-        float* dst = a.dqt + ((b * a.Hq + h) * D + ch * 128 + lt) * static_cast<long long>(a.Sq) +
-                     static_cast<long long>(m) * AB_BQ;
-#pragma unroll 1
-        for (int c0 = wg * 32; c0 < AB_BQ; c0 += 64) {
-          uint32_t r[32];
-          tmem_ld_32x32(tmem + C::TC_DQ + ch * AB_BQ + c0, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            red_add_v4_f32(dst + c0 + i, __uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]),
-                           __uint_as_float(r[i + 3]));
-        }
-      }
+      tmem_st_wait();
       tc_fence_before();
-      __syncthreads();   // dQ^T columns are reused by the next step
-      tc_fence_after();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_a2);
     }
-  }
-  if (!ok && tid == 0) {   // leave no copy in flight
-    int dummy = 0;
-    mbar_wait_bounded(&bar_q[0], 0, &dummy);
-    mbar_wait_bounded(&bar_q[1], 0, &dummy);
-  }
-  if (ok) {
-    const long long orow = ((b * a.Skv + k0 + lt) * a.Hkv + hk) * D;
-#pragma unroll 1
-    for (int which = 0; which < 2; ++which) {
-      if ((which == 0 && !C::NEED_PT) || (which == 1 && !C::NEED_DS)) continue;
-      __nv_bfloat16* dst = (which == 0 ? a.dv : a.dk) + orow;
-      const uint32_t tc = which == 0 ? C::TC_DV : C::TC_DK;
-#pragma unroll 1
-      for (int c0 = wg * 32; c0 < D; c0 += 64) {
-        uint32_t o[32];
-        if (steps > 0) {
-          tmem_ld_32x32(tmem + tc + c0, o);
-          tmem_ld_wait();
-        } else {
+    const long long row_pos = (C::ROWQ ? a.q_pos0 : a.k_pos0) + ri;
+    for (int j = 0; j < steps && ok; ++j) {
+      const int col0 = (c_begin + j % per_head) * AB_STEP + wg * 32;   // first column of this thread's half
+      if (!C::ROWQ) {   // the scalars of this half's queries, one copy per warp: no barrier between warps
+        const int qi = col0 + lane;
+        const long long i = (static_cast<long long>(b) * a.Hq + hq0 + j / per_head) * a.Sq + qi;
+        const float l2 = qi < a.Sq ? lse2_of(a.lse[i]) : INFINITY;
+        const float dl = C::HAS_DP && qi < a.Sq ? a.delta[i] : 0.f;
+        __syncwarp();
+        v_lse2[lane] = l2;
+        v_delta[lane] = dl;
+        __syncwarp();
+      }
+      if (!wait(bar_sd, j & 1)) break;
+      tc_fence_after();
+      uint32_t rs[32], rp[32];
+      tmem_ld_32x32(tmem + C::TC_S + wg * 32, rs);
+      if (C::HAS_DP) tmem_ld_32x32(tmem + C::TC_DP + wg * 32, rp);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_free);
+      uint32_t pk[16], dk[16];
+      auto form = [&](auto masked, int lo, int hi) {
+        constexpr bool MASKED = decltype(masked)::value;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 0u;
-        }
+        for (int i = 0; i < 32; i += 4) {
+          float4 l2, dl;
+          if (C::ROWQ) {
+            l2 = make_float4(row_lse2, row_lse2, row_lse2, row_lse2);
+            dl = make_float4(row_delta, row_delta, row_delta, row_delta);
+          } else {
+            l2 = *reinterpret_cast<const float4*>(v_lse2 + i);
+            if (C::HAS_DP) dl = *reinterpret_cast<const float4*>(v_delta + i);
+          }
+          const float l2v[4] = {l2.x, l2.y, l2.z, l2.w}, dlv[4] = {dl.x, dl.y, dl.z, dl.w};
+          float p[4], ds[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint4 u;
-          u.x = pack_bf16x2(__uint_as_float(o[8 * c + 0]), __uint_as_float(o[8 * c + 1]));
-          u.y = pack_bf16x2(__uint_as_float(o[8 * c + 2]), __uint_as_float(o[8 * c + 3]));
-          u.z = pack_bf16x2(__uint_as_float(o[8 * c + 4]), __uint_as_float(o[8 * c + 5]));
-          u.w = pack_bf16x2(__uint_as_float(o[8 * c + 6]), __uint_as_float(o[8 * c + 7]));
-          *reinterpret_cast<uint4*>(dst + c0 + 8 * c) = u;
+          for (int e = 0; e < 4; ++e) {
+            p[e] = exp2f(__uint_as_float(rs[i + e]) * a.scale_log2 - l2v[e]);
+            if (MASKED && (i + e < lo || i + e >= hi)) p[e] = 0.f;
+            if (C::HAS_DP) ds[e] = p[e] * (__uint_as_float(rp[i + e]) - dlv[e]) * a.scale;
+          }
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) {
+            if (C::ACC_V) pk[(i + e) / 2] = pack_bf16x2(p[e], p[e + 1]);
+            if (C::ACC_1) dk[(i + e) / 2] = pack_bf16x2(ds[e], ds[e + 1]);
+          }
         }
+      };
+      // columns [lo, hi) of this half are visible from this row; most steps are visible from every row of the warp
+      int lo = 0, hi = 32;
+      if (C::ROWQ) {
+        long long v = a.Skv - col0;
+        if (a.causal) v = min(v, row_pos - (a.k_pos0 + col0) + 1);
+        hi = static_cast<int>(max(min(v, 32ll), 0ll));
+      } else if (a.causal) {
+        lo = static_cast<int>(max(min(row_pos - (a.q_pos0 + col0), 32ll), 0ll));
+      }
+      if (__any_sync(0xffffffffu, lo > 0 || hi < 32)) form(std::true_type{}, lo, hi);
+      else form(std::false_type{}, lo, hi);
+      if (j > 0 && !wait(bar_acc, (j - 1) & 1)) break;   // the previous step has read the buffers
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint32_t off = asw128(row, wg * 4 + c);
+        if (C::ACC_V)
+          *reinterpret_cast<uint4*>(smem + C::PT + off) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+        if (C::ACC_1)
+          *reinterpret_cast<uint4*>(smem + C::DS + off) = make_uint4(dk[4 * c], dk[4 * c + 1], dk[4 * c + 2], dk[4 * c + 3]);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_ds);
+    }
+    if (ok && steps > 0) wait(bar_acc, (steps - 1) & 1);
+    if (ok) {
+      tc_fence_after();
+      // accumulators as bf16 over operands that are no longer read, then out by TMA, which drops rows past the end
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        if ((which == 0 && !C::ACC_1) || (which == 1 && !C::ACC_V)) continue;
+        uint8_t* stage = smem + (which == 0 ? C::A1 : C::STG_V);
+        const uint32_t tc = which == 0 ? C::TC_1 : C::TC_V;
+#pragma unroll 1
+        for (int c0 = wg * 32; c0 < D; c0 += 64) {
+          uint32_t o[32];
+          if (steps > 0) {
+            tmem_ld_32x32(tmem + tc + c0, o);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = 0u;
+          }
+          uint8_t* box = stage + (c0 >> 6) * 16384;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint4 u;
+            u.x = pack_bf16x2(__uint_as_float(o[8 * c + 0]), __uint_as_float(o[8 * c + 1]));
+            u.y = pack_bf16x2(__uint_as_float(o[8 * c + 2]), __uint_as_float(o[8 * c + 3]));
+            u.z = pack_bf16x2(__uint_as_float(o[8 * c + 4]), __uint_as_float(o[8 * c + 5]));
+            u.w = pack_bf16x2(__uint_as_float(o[8 * c + 6]), __uint_as_float(o[8 * c + 7]));
+            *reinterpret_cast<uint4*>(box + asw128(row, wg * 4 + c)) = u;
+          }
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_out);
+      if (tid == 64 && mbar_wait_bounded(bar_out, 0, abort_flag)) {
+#pragma unroll
+        for (int c = 0; c < NB; ++c) {
+          if (C::ACC_1) tma_store_3d(&tmO1, smem + C::A1 + c * 16384, head * D + c * 64, r0, b);
+          if (C::ACC_V) tma_store_3d(&tmOV, smem + C::STG_V + c * 16384, head * D + c * 64, r0, b);
+        }
+        tma_store_commit();
+        tma_store_wait_read();
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (tid < 32) {
+  if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -838,26 +958,9 @@ attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16*
   }
 }
 
-// dq[b, q, h, d] (bf16) = dqt[b, h, d, q] (fp32): 32 x 32 tiles through shared memory
-__global__ void __launch_bounds__(256)
-attention_dq_transpose_kernel(const float* __restrict__ dqt, __nv_bfloat16* __restrict__ dq, int Sq, int Hq, int D) {
-  __shared__ float tile[32][33];
-  const long long bh = blockIdx.z;
-  const long long b = bh / Hq, h = bh % Hq;
-  const int q0 = blockIdx.x * 32, d0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8
-  const float* src = dqt + (bh * D + d0) * static_cast<long long>(Sq) + q0;
-#pragma unroll
-  for (int r = ty; r < 32; r += 8) tile[r][tx] = src[static_cast<long long>(r) * Sq + tx];   // [d][q]
-  __syncthreads();
-#pragma unroll
-  for (int r = ty; r < 32; r += 8)
-    dq[((b * Sq + q0 + r) * Hq + h) * D + d0 + tx] = __float2bfloat16_rn(tile[tx][r]);
-}
-
 template <int D, int MODE>
-static int launch_bwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-                      const AttBwdArgs& a, long long B, cudaStream_t st) {
+static int launch_bwd(const CUtensorMap& a1, const CUtensorMap& a2, const CUtensorMap& b1, const CUtensorMap& b2,
+                      const CUtensorMap& o1, const CUtensorMap& ov, const AttBwdArgs& a, cudaStream_t st) {
   using C = AttBwdCfg<D, MODE>;
   static bool attr = false;
   if (!attr) {
@@ -866,44 +969,52 @@ static int launch_bwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtens
       return -11;
     attr = true;
   }
-  dim3 grid(static_cast<unsigned>((a.Skv / AB_BKV) * a.Hkv * B));
-  attention_bwd_kernel<D, MODE><<<grid, AB_THREADS, C::BYTES, st>>>(mq, mk, mv, mdo, a);
+  const long long blocks =
+      static_cast<long long>(((C::ROWQ ? a.Sq : a.Skv) + AB_ROWS - 1) / AB_ROWS) * (C::ROWQ ? a.Hq : a.Hkv) * a.B;
+  if (blocks > 0x7fffffffLL) return -2;
+  attention_bwd_kernel<D, MODE><<<static_cast<unsigned>(blocks), AB_THREADS, C::BYTES, st>>>(a1, a2, b1, b2, o1, ov, a);
   return static_cast<int>(cudaGetLastError());
 }
 
 // q, o, d_o: bf16 [B, Sq, Hq, D]; k, v: bf16 [B, Skv, Hkv, D]; lse: fp32 [B, Hq, Sq] from the forward.
-// Scratch: delta fp32 [B, Hq, Sq]; dqt fp32 [B, Hq, D, Sq], zeroed by the caller.
+// Scratch: delta fp32 [B, Hq, Sq].
 // Outputs: dq bf16 [B, Sq, Hq, D]; dk, dv bf16 [B, Skv, Hkv, D] (summed over the query heads of each GQA group).
-// Sq % 64 == 0, Skv % 128 == 0.
 extern "C" int cvb_attention_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                                 const float* lse, float* delta, float* dqt, void* dq, void* dk, void* dv, long long B,
-                                 int Sq, int Skv, int Hq, int Hkv, int D, float scale, int causal, long long q_pos0,
+                                 const float* lse, float* delta, void* dq, void* dk, void* dv, long long B, int Sq,
+                                 int Skv, int Hq, int Hkv, int D, float scale, int causal, long long q_pos0,
                                  long long k_pos0, int* status, void* stream) {
   if (B <= 0 || Sq <= 0 || Skv <= 0) return 0;
-  if (Sq % AB_BQ || Skv % AB_BKV || Hkv <= 0 || Hq % Hkv || !(scale > 0.f) || (D != 128 && D != 256)) return -1;
+  if (Hkv <= 0 || Hq % Hkv || !(scale > 0.f) || (D != 128 && D != 256)) return -1;
   if (B * Sq > 0x7fffffffLL || B * Skv > 0x7fffffffLL) return -2;
+  for (const void* p : {q, k, v, o, d_o, static_cast<const void*>(dq), static_cast<const void*>(dk),
+                        static_cast<const void*>(dv)})
+    if (reinterpret_cast<uintptr_t>(p) & 15) return -3;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  CUtensorMap mq, mk, mv, mdo;
   const uint64_t qc = static_cast<uint64_t>(Hq) * D, kc = static_cast<uint64_t>(Hkv) * D;
-  if (make_tensor_map_2d(&mq, q, 2, qc, B * Sq, qc * 2, 64, 64) || make_tensor_map_2d(&mdo, d_o, 2, qc, B * Sq, qc * 2, 64, 64) ||
-      make_tensor_map_2d(&mk, k, 2, kc, B * Skv, kc * 2, 64, 128) || make_tensor_map_2d(&mv, v, 2, kc, B * Skv, kc * 2, 64, 128))
+  auto map = [&](CUtensorMap* m, const void* p, bool query, uint32_t box) {
+    const uint64_t cols = query ? qc : kc, rows = query ? Sq : Skv;
+    return make_tensor_map_3d(m, p, 2, cols, rows, B, cols * 2, cols * 2 * rows, 64, box);
+  };
+  CUtensorMap q128, q64, k128, k64, v128, v64, do128, do64, mdq, mdk, mdv;
+  if (map(&q128, q, true, 128) || map(&q64, q, true, 64) || map(&do128, d_o, true, 128) || map(&do64, d_o, true, 64) ||
+      map(&k128, k, false, 128) || map(&k64, k, false, 64) || map(&v128, v, false, 128) || map(&v64, v, false, 64) ||
+      map(&mdq, dq, true, 128) || map(&mdk, dk, false, 128) || map(&mdv, dv, false, 128))
     return -10;
   const long long rows = B * Sq * Hq;
   attention_delta_kernel<<<static_cast<unsigned>((rows * 32 + 255) / 256), 256, 0, st>>>(
       static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, B, Sq, Hq, D);
   AttBwdArgs a{};
-  a.lse = lse; a.delta = delta; a.dk = static_cast<__nv_bfloat16*>(dk); a.dv = static_cast<__nv_bfloat16*>(dv);
-  a.dqt = dqt; a.Sq = Sq; a.Skv = Skv; a.Hq = Hq; a.Hkv = Hkv; a.B = static_cast<int>(B); a.scale = scale;
-  a.scale_log2 = scale * 1.4426950408889634f; a.causal = causal; a.q_pos0 = q_pos0; a.k_pos0 = k_pos0; a.status = status;
+  a.lse = lse; a.delta = delta; a.Sq = Sq; a.Skv = Skv; a.Hq = Hq; a.Hkv = Hkv; a.B = static_cast<int>(B);
+  a.scale = scale; a.scale_log2 = scale * 1.4426950408889634f; a.causal = causal; a.q_pos0 = q_pos0; a.k_pos0 = k_pos0;
+  a.status = status;
   int rc;
   if (D == 128) {
-    rc = launch_bwd<128, 0>(mq, mk, mv, mdo, a, B, st);
+    rc = launch_bwd<128, BWD_KV>(k128, v128, q64, do64, mdk, mdv, a, st);
+    if (rc == 0) rc = launch_bwd<128, BWD_Q>(q128, do128, k64, v64, mdq, mdq, a, st);
   } else {
-    rc = launch_bwd<256, 1>(mq, mk, mv, mdo, a, B, st);
-    if (rc == 0) rc = launch_bwd<256, 2>(mq, mk, mv, mdo, a, B, st);
+    rc = launch_bwd<256, BWD_V>(k128, v128, q64, do64, mdv, mdv, a, st);
+    if (rc == 0) rc = launch_bwd<256, BWD_K>(k128, v128, q64, do64, mdk, mdk, a, st);
+    if (rc == 0) rc = launch_bwd<256, BWD_Q>(q128, do128, k64, v64, mdq, mdq, a, st);
   }
-  if (rc != 0) return rc;
-  dim3 tg(Sq / 32, D / 32, static_cast<unsigned>(B * Hq));
-  attention_dq_transpose_kernel<<<tg, 256, 0, st>>>(dqt, static_cast<__nv_bfloat16*>(dq), Sq, Hq, D);
-  return static_cast<int>(cudaGetLastError());
+  return rc;
 }

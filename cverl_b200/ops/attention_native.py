@@ -47,16 +47,15 @@ def _bwd(q4, k4, v4, out, lse, dout, scale, causal, q_pos0, k_pos0):
     Skv, Hkv = k4.shape[1], k4.shape[2]
     dev = q4.device
     delta = torch.empty((B, Hq, Sq), dtype=torch.float32, device=dev)
-    dqt = torch.zeros((B, Hq, D, Sq), dtype=torch.float32, device=dev)
     dq = torch.empty_like(q4)
     dk = torch.empty((B, Skv, Hkv, D), dtype=torch.bfloat16, device=dev)   # summed over each GQA group in-kernel
     dv = torch.empty((B, Skv, Hkv, D), dtype=torch.bfloat16, device=dev)
     rc = nv.cuda().cvb_attention_bwd(q4.data_ptr(), k4.data_ptr(), v4.data_ptr(), out.data_ptr(), dout.data_ptr(),
-                                     lse.data_ptr(), delta.data_ptr(), dqt.data_ptr(), dq.data_ptr(), dk.data_ptr(),
-                                     dv.data_ptr(), B, Sq, Skv, Hq, Hkv, D, scale, int(causal), q_pos0, k_pos0,
+                                     lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                                     B, Sq, Skv, Hq, Hkv, D, scale, int(causal), q_pos0, k_pos0,
                                      nv.status_word(dev).data_ptr(), nv.stream())
     nv.check(rc, "cvb_attention_bwd")
-    count_launch(4 if D == 128 else 5)
+    count_launch(3 if D == 128 else 4)
     return dq, dk, dv
 
 

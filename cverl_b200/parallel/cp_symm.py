@@ -106,17 +106,23 @@ def ring_backward(ctx, do):
     lib = nv.cuda()
     for owner in range(cp_rank, -1, -1):
         delta = torch.empty((B, Hq, L), dtype=torch.float32, device=q4.device)
-        dqt = torch.zeros((B, Hq, D, L), dtype=torch.float32, device=q4.device)
+        kp, vp = bk.peer_ptrs[owner], bv.peer_ptrs[owner]
+        if owner != cp_rank:
+            # every query tile of the dQ kernel walks all keys: the peer's K and V cross the link once, into local memory
+            k_l, v_l = (torch.empty(kshape, dtype=torch.bfloat16, device=q4.device) for _ in range(2))
+            for dst, src in ((k_l, kp), (v_l, vp)):
+                nv.check(lib.cvb_device_memcpy_async(dst.data_ptr(), src, dst.numel() * 2, nv.stream()), "cp K|V copy")
+            kp, vp = k_l.data_ptr(), v_l.data_ptr()
         dq_h = torch.empty_like(q4)
         dkh = torch.empty((B, L, Hkv, D), dtype=torch.bfloat16, device=q4.device)
         dvh = torch.empty((B, L, Hkv, D), dtype=torch.bfloat16, device=q4.device)
-        rc = lib.cvb_attention_bwd(q4.data_ptr(), bk.peer_ptrs[owner], bv.peer_ptrs[owner], out.data_ptr(),
-                                   do4.data_ptr(), lse.data_ptr(), delta.data_ptr(), dqt.data_ptr(), dq_h.data_ptr(),
+        rc = lib.cvb_attention_bwd(q4.data_ptr(), kp, vp, out.data_ptr(),
+                                   do4.data_ptr(), lse.data_ptr(), delta.data_ptr(), dq_h.data_ptr(),
                                    dkh.data_ptr(), dvh.data_ptr(), B, L, L, Hq, Hkv, D, scale, int(owner == cp_rank),
                                    cp_rank * shard_len, owner * shard_len, nv.status_word(q4.device).data_ptr(),
                                    nv.stream())
         nv.check(rc, "cvb_attention_bwd (peer pull)")
-        count_launch(5)
+        count_launch(3 if D == 128 else 4)
         dq += dq_h.float()
         stage[owner, 0] = dkh.float()
         stage[owner, 1] = dvh.float()

@@ -57,3 +57,29 @@ def test_forward_scores_that_grow_along_the_keys():
         out, _ = an._fwd(q, k, v, 1.0 / math.sqrt(D), True, 0, 0)
         want, _ = _ref(q, k, v, 1.0 / math.sqrt(D), True, 0, 0)
         assert (out.double() - want).norm() <= 2.0 ** -8 * want.norm()
+
+
+@pytest.mark.parametrize("D,Hq,Hkv", [(128, 4, 1), (128, 2, 2), (256, 2, 2), (256, 4, 1)])
+@pytest.mark.parametrize("Sq,Skv,causal,q0,k0", [
+    (1, 1, True, 0, 0), (63, 63, True, 0, 0), (65, 65, True, 0, 0), (128, 128, True, 0, 0), (129, 129, True, 0, 0),
+    (640, 640, True, 0, 0), (1001, 1001, True, 0, 0),
+    (200, 333, False, 0, 0), (384, 384, True, 0, 100), (256, 128, True, 500, 0), (130, 130, True, 0, 1000)])
+def test_backward_edges(D, Hq, Hkv, Sq, Skv, causal, q0, k0):
+    from cverl_b200 import _native as nv
+    from cverl_b200.ops import attention_native as an
+    q, k, v = _inputs(2, Sq, Skv, Hq, Hkv, D, Sq + Skv + 1)
+    do = _inputs(2, Sq, Skv, Hq, Hkv, D, 99)[0]
+    scale = 1 / math.sqrt(D)
+    out, lse = an._fwd(q, k, v, scale, causal, q0, k0)
+    got = an._bwd(q, k, v, out, lse, do, scale, causal, q0, k0)
+    again = an._bwd(q, k, v, out, lse, do, scale, causal, q0, k0)
+    nv.check_status()
+    leaves = [t.double().requires_grad_(True) for t in (q, k, v)]
+    want, _ = _ref(*leaves, scale, causal, q0, k0)
+    grads = torch.autograd.grad(want, leaves, do.double())
+    for name, a, b, r in zip("qkv", got, again, grads):
+        assert torch.equal(a, b), name           # no sums across CTAs: the order is fixed
+        # P, dS, the saved output behind Delta and the result are rounded to bf16, 2^-9 each; with one visible key
+        # dq and dk cancel to zero, and what is left is the rounding of dP - Delta, of the size of |dO| |V| scale
+        floor = 2.0 ** -8 * scale * float(do.double().norm()) * D ** 0.5 if Skv < 8 and name != "v" else 0.0
+        assert (a.double() - r).norm() <= 4 * 2.0 ** -9 * r.norm() + floor + 1e-9, name
