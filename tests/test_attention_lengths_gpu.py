@@ -59,6 +59,19 @@ def test_forward_scores_that_grow_along_the_keys():
         assert (out.double() - want).norm() <= 2.0 ** -8 * want.norm()
 
 
+@pytest.mark.parametrize("D", [128, 256])
+@pytest.mark.parametrize("S", [640, 1500])
+def test_forward_scores_that_grow_now_and_then(D, S):
+    """Wide scores: a row's maximum passes the rescale bound at irregular blocks, with blocks in between that do not."""
+    from cverl_b200.ops import attention_native as an
+    q, k, v = _inputs(2, S, S, 2, 1, D, 11)
+    q = (q.float() * 12).to(torch.bfloat16)
+    out, lse = an._fwd(q, k, v, 1.0 / math.sqrt(D), True, 0, 0)
+    want, lse_want = _ref(q, k, v, 1.0 / math.sqrt(D), True, 0, 0)
+    assert (out.double() - want).norm() <= 2.0 ** -8 * want.norm()
+    assert (lse.double() - lse_want).abs().max() < 1e-3      # |score| up to 60: 2^-24 relative in fp32, with margin
+
+
 @pytest.mark.parametrize("D,Hq,Hkv", [(128, 4, 1), (128, 2, 2), (256, 2, 2), (256, 4, 1)])
 @pytest.mark.parametrize("Sq,Skv,causal,q0,k0", [
     (1, 1, True, 0, 0), (63, 63, True, 0, 0), (65, 65, True, 0, 0), (128, 128, True, 0, 0), (129, 129, True, 0, 0),
