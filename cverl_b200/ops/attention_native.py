@@ -21,12 +21,22 @@ def _enabled() -> bool:
 
 
 def supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, seq: int) -> bool:
-    """bf16, head dim 128 or 256, sequence length a multiple of 128 (query blocks of 128, key blocks of 128)."""
+    """bf16, head dim 256 at any sequence length, head dim 128 at multiples of 128.
+
+    The kernels take any length at both head dims.  At 128 and other lengths the library's kernel is the faster one
+    (forward and backward of 4 x 1500, 32 / 4 heads: 430 us against about 660 for 4 x 1536 here); at 256 it is not (8 x 1088,
+    8 / 2 heads: 601 us in the library, 416 here)."""
     if not (_enabled() and q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16):
         return False
     d = q.shape[-1]
-    return d in (128, 256) and v.shape[-1] == d and k.shape[-1] == d and seq % 128 == 0 and \
+    return d in (128, 256) and v.shape[-1] == d and k.shape[-1] == d and (seq % 128 == 0 or d == 256) and \
         q.shape[-2] % k.shape[-2] == 0
+
+
+def _operand(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous, on a 16-byte boundary (TMA)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def _fwd(q4, k4, v4, scale, causal, q_pos0, k_pos0):
@@ -65,7 +75,7 @@ class _AttentionBlock(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q4, k4, v4, scale, causal, q_pos0, k_pos0):
-        q4, k4, v4 = q4.contiguous(), k4.contiguous(), v4.contiguous()
+        q4, k4, v4 = _operand(q4), _operand(k4), _operand(v4)
         out, lse = _fwd(q4, k4, v4, scale, causal, q_pos0, k_pos0)
         ctx.save_for_backward(q4, k4, v4, out, lse)
         ctx.cfg = (scale, causal, q_pos0, k_pos0)
@@ -76,7 +86,7 @@ class _AttentionBlock(torch.autograd.Function):
     def backward(ctx, dout, _dlse):
         q4, k4, v4, out, lse = ctx.saved_tensors
         scale, causal, q_pos0, k_pos0 = ctx.cfg
-        dq, dk, dv = _bwd(q4, k4, v4, out, lse, dout.contiguous(), scale, causal, q_pos0, k_pos0)
+        dq, dk, dv = _bwd(q4, k4, v4, out, lse, _operand(dout), scale, causal, q_pos0, k_pos0)
         return dq, dk, dv, None, None, None, None
 
 
