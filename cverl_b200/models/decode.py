@@ -27,6 +27,7 @@ import torch.nn.functional as F
 
 from .. import ops
 from ..ops.gdn import l2norm
+from ..ops.gemm import use_native
 from ..ops.norm import apply_rope_ref, rmsnorm_ref
 
 
@@ -80,7 +81,12 @@ def _tp_sum(model, t: torch.Tensor) -> torch.Tensor:
 
 def _full_logits(model, hidden: torch.Tensor) -> torch.Tensor:
     """hidden [B, H] -> fp32 logits [B, V]; the LM head is sharded over vocabulary rows under tensor parallelism."""
-    logits = hidden.float() @ model.lm_head_weight().float().t()
+    w = model.lm_head_weight()
+    if hidden.dtype == w.dtype == torch.bfloat16 and use_native(hidden):
+        # bf16 products summed in fp32, as after a conversion of both to fp32, without the converted copy of the head
+        logits = ops.gemm_nt(hidden, w, out_dtype=torch.float32)
+    else:
+        logits = hidden.float() @ w.float().t()
     if model.ctx.tp_size > 1:
         import torch.distributed as dist
         parts = [torch.empty_like(logits) for _ in range(model.ctx.tp_size)]
