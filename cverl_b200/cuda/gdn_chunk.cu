@@ -29,6 +29,13 @@ __device__ __forceinline__ uint32_t csw128(uint32_t row, uint32_t chunk) {
   return row * 128u + ((chunk ^ (row & 7u)) << 4);
 }
 
+__device__ __forceinline__ void fma4(float4& acc, float x, const float4& b) {
+  acc.x += x * b.x;
+  acc.y += x * b.y;
+  acc.z += x * b.z;
+  acc.w += x * b.w;
+}
+
 struct PrepArgs {
   const float* beta;   // [B, T, H]
   const float* g;      // [B, T, H]
@@ -110,12 +117,16 @@ gdn_chunk_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
-  if (tid == 0) {  // inclusive scan of g
-    float acc = 0.f;
-    for (int t = 0; t < CC; ++t) {
-      acc += s_c[t];
-      s_c[t] = acc;
+  if (warp == 0) {  // inclusive scan of g, two neighbouring tokens per lane
+    const float g0 = s_c[2 * tid], g1 = s_c[2 * tid + 1];
+    float incl = g0 + g1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (tid >= o) incl += up;
     }
+    s_c[2 * tid] = incl - g1;
+    s_c[2 * tid + 1] = incl;
   }
   bool ok = mbar_wait_bounded(bar_load, 0, abort_flag);
   if (!ok) {
@@ -142,8 +153,10 @@ gdn_chunk_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     float sk = 0.f, sq = 0.f;
 #pragma unroll
     for (int ch = 0; ch < 8; ++ch) {
-      const uint4 ku = *reinterpret_cast<const uint4*>(kb + ch * 16);
-      const uint4 qu = *reinterpret_cast<const uint4*>(qb + ch * 16);
+      // rows lie 128 bytes apart: every thread starts at another of the row's 16-byte pieces, all hit the same banks
+      // otherwise
+      const uint4 ku = *reinterpret_cast<const uint4*>(kb + ((ch ^ (t & 7)) << 4));
+      const uint4 qu = *reinterpret_cast<const uint4*>(qb + ((ch ^ (t & 7)) << 4));
       const __nv_bfloat162* kp = reinterpret_cast<const __nv_bfloat162*>(&ku);
       const __nv_bfloat162* qp = reinterpret_cast<const __nv_bfloat162*>(&qu);
 #pragma unroll
@@ -235,32 +248,49 @@ gdn_chunk_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     __syncthreads();
 #pragma unroll 1
     for (int i = 1; i < 4; ++i) {
-      for (int e = tid; e < i * 256; e += CTHREADS) {
-        const int jb = e >> 8, r = (e >> 4) & 15, c = e & 15;
-        float acc0 = 0.f, acc1 = 0.f;
+      // four columns per thread: five 16-byte reads for 16 FMAs (one column: 8 4-byte reads for 4)
+      const float4* A4 = reinterpret_cast<const float4*>(Am);
+      float4* X4 = reinterpret_cast<float4*>(Xs);
+      for (int e = tid; e < i * 64; e += CTHREADS) {
+        const int jb = e >> 6, r = 16 * i + ((e >> 2) & 15), cq = e & 3;
+        float4 acc0 = make_float4(0.f, 0.f, 0.f, 0.f), acc1 = acc0;
         for (int k = jb; k < i; ++k) {
 #pragma unroll
-          for (int m = 0; m < 16; m += 2) {
-            acc0 += am(16 * i + r, 16 * k + m) * am(16 * k + m, 16 * jb + c);
-            acc1 += am(16 * i + r, 16 * k + m + 1) * am(16 * k + m + 1, 16 * jb + c);
+          for (int mq = 0; mq < 4; ++mq) {
+            const float4 x = A4[r * 16 + ((4 * k + mq) ^ (r & 15))];
+            const int m = 16 * k + 4 * mq, col = 4 * jb + cq;
+            fma4(acc0, x.x, A4[m * 16 + (col ^ (m & 15))]);
+            fma4(acc1, x.y, A4[(m + 1) * 16 + (col ^ ((m + 1) & 15))]);
+            fma4(acc0, x.z, A4[(m + 2) * 16 + (col ^ ((m + 2) & 15))]);
+            fma4(acc1, x.w, A4[(m + 3) * 16 + (col ^ ((m + 3) & 15))]);
           }
         }
-        Xs[e] = acc0 + acc1;
+        X4[e] = make_float4(acc0.x + acc1.x, acc0.y + acc1.y, acc0.z + acc1.z, acc0.w + acc1.w);
       }
       __syncthreads();
-      for (int e = tid; e < i * 256; e += CTHREADS) {
-        const int jb = e >> 8, r = (e >> 4) & 15, c = e & 15;
-        float acc0 = 0.f, acc1 = 0.f;
+      for (int e = tid; e < i * 64; e += CTHREADS) {
+        const int jb = e >> 6, r = 16 * i + ((e >> 2) & 15), cq = e & 3;
+        float4 acc0 = make_float4(0.f, 0.f, 0.f, 0.f), acc1 = acc0;
 #pragma unroll
-        for (int m = 0; m < 16; m += 2) {   // T_ii is lower triangular: its upper entries are stored zeros
-          acc0 += am(16 * i + r, 16 * i + m) * Xs[(jb << 8) + (m << 4) + c];
-          acc1 += am(16 * i + r, 16 * i + m + 1) * Xs[(jb << 8) + ((m + 1) << 4) + c];
+        for (int mq = 0; mq < 4; ++mq) {   // T_ii is lower triangular: its upper entries are stored zeros
+          const float4 x = A4[r * 16 + ((4 * i + mq) ^ (r & 15))];
+          const float4* xk = X4 + (jb << 6) + (mq << 4) + cq;
+          fma4(acc0, x.x, xk[0]);
+          fma4(acc1, x.y, xk[4]);
+          fma4(acc0, x.z, xk[8]);
+          fma4(acc1, x.w, xk[12]);
         }
-        am(16 * i + r, 16 * jb + c) = -(acc0 + acc1);
+        reinterpret_cast<float4*>(Am)[r * 16 + ((4 * jb + cq) ^ (r & 15))] =
+            make_float4(-(acc0.x + acc1.x), -(acc0.y + acc1.y), -(acc0.z + acc1.z), -(acc0.w + acc1.w));
       }
       __syncthreads();
     }
   }
+  if (tid < CC) {   // the row factors of step 4, while they are still spread over both halves of the block
+    s_pk[tid] = __expf(s_c[CC - 1] - s_c[tid]) * s_rk[tid];
+    s_pq[tid] = __expf(s_c[tid]) * s_rq[tid];
+  }
+  __syncthreads();
   if (tid < CC) {
     // column j of T into registers, then the scaled bf16 operand tiles (they overwrite A) and the fp32 copy
     const int j = tid;
@@ -285,32 +315,28 @@ gdn_chunk_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int r = 0; r < CC; ++r) a.Tm[(item * CC + r) * CC + j] = col[r];
     }
   } else {
-    // 4. Kd = e^{c_C - c_t} rk_t k_t and Qd = e^{c_t} rq_t q_t, one row per thread
+    // 4. Kd = e^{c_C - c_t} rk_t k_t and Qd = e^{c_t} rq_t q_t, 16 threads per 256-byte row
     const int t = tid - CC;
-    const float fk = __expf(s_c[CC - 1] - s_c[t]) * s_rk[t];
-    const float fq = __expf(s_c[t]) * s_rq[t];
-    __nv_bfloat16* kd = a.Kd + (item * CC + t) * CD;
-    __nv_bfloat16* qd = a.Qd + (item * CC + t) * CD;
+    uint4* kd = reinterpret_cast<uint4*>(a.Kd + item * CC * CD);
+    uint4* qd = reinterpret_cast<uint4*>(a.Qd + item * CC * CD);
+#pragma unroll 4
+    for (int idx = t; idx < CC * 16; idx += 64) {
+      const int row = idx >> 4, hb = (idx >> 3) & 1, ch = idx & 7;
+      const float fk = s_pk[row], fq = s_pq[row];
+      const uint8_t* kb = smem + PrepSmem::KQ + hb * 16384 + csw128(row, ch);
+      const uint4 ku = *reinterpret_cast<const uint4*>(kb);
+      const uint4 qu = *reinterpret_cast<const uint4*>(kb + 8192);
+      const __nv_bfloat162* kp = reinterpret_cast<const __nv_bfloat162*>(&ku);
+      const __nv_bfloat162* qp = reinterpret_cast<const __nv_bfloat162*>(&qu);
+      uint32_t ko[4], qo[4];
 #pragma unroll
-    for (int hb = 0; hb < 2; ++hb) {
-      const uint8_t* kb = smem + PrepSmem::KQ + hb * 16384;
-      const uint8_t* qb = kb + 8192;
-#pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
-        const uint4 ku = *reinterpret_cast<const uint4*>(kb + csw128(t, ch));
-        const uint4 qu = *reinterpret_cast<const uint4*>(qb + csw128(t, ch));
-        const __nv_bfloat162* kp = reinterpret_cast<const __nv_bfloat162*>(&ku);
-        const __nv_bfloat162* qp = reinterpret_cast<const __nv_bfloat162*>(&qu);
-        uint32_t ko[4], qo[4];
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          const float2 kf = __bfloat1622float2(kp[jj]), qf = __bfloat1622float2(qp[jj]);
-          ko[jj] = pack_bf16x2(kf.x * fk, kf.y * fk);
-          qo[jj] = pack_bf16x2(qf.x * fq, qf.y * fq);
-        }
-        *reinterpret_cast<uint4*>(kd + hb * 64 + ch * 8) = make_uint4(ko[0], ko[1], ko[2], ko[3]);
-        *reinterpret_cast<uint4*>(qd + hb * 64 + ch * 8) = make_uint4(qo[0], qo[1], qo[2], qo[3]);
+      for (int jj = 0; jj < 4; ++jj) {
+        const float2 kf = __bfloat1622float2(kp[jj]), qf = __bfloat1622float2(qp[jj]);
+        ko[jj] = pack_bf16x2(kf.x * fk, kf.y * fk);
+        qo[jj] = pack_bf16x2(qf.x * fq, qf.y * fq);
       }
+      kd[idx] = make_uint4(ko[0], ko[1], ko[2], ko[3]);
+      qd[idx] = make_uint4(qo[0], qo[1], qo[2], qo[3]);
     }
     if (t == 0) a.egam[item] = __expf(s_c[CC - 1]);
     if (a.aux) {
