@@ -29,7 +29,11 @@ namespace cvb {
 
 constexpr int GC = 64;    // chunk length
 constexpr int GD = 128;   // dk = dv
-constexpr int GTHREADS = 128;
+// Two warpgroups: warps w and w + 4 share TMEM lane quadrant w (the same 32 rows of the state) and take every second
+// 32-column chunk of each TMEM -> register pass.  The scan is one serial chain per sequence, and those passes are its
+// longest links: 16 sequences of 1280 x 16 heads took 133 us forward and 135 us backward with one warpgroup,
+// 121 and 131 us with two (what is left is mostly the MMA and barrier latency of 20 chunks in a row).
+constexpr int GTHREADS = 256;
 
 // byte offset of 16-byte chunk `chunk` of row `row` in a 128-byte-swizzled tile with 128-byte rows
 __device__ __forceinline__ uint32_t sw128(uint32_t row, uint32_t chunk) {
@@ -80,9 +84,9 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* m, ui
 
 // S^T (or dS^T) round trip: TMEM -> (global bf16, smem bf16 operand) -> scaled -> TMEM
 __device__ __forceinline__ void state_round_trip(uint32_t t_state, uint8_t* s_op, __nv_bfloat16* g_row,
-                                                 float scale, int v) {
+                                                 float scale, int v, int wg) {
 #pragma unroll 1
-  for (int c0 = 0; c0 < GD; c0 += 32) {
+  for (int c0 = wg * 32; c0 < GD; c0 += 64) {
     uint32_t r[32];
     tmem_ld_32x32(t_state + c0, r);
     tmem_ld_wait();
@@ -143,18 +147,20 @@ gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   uint64_t *bar_w = bars, *bar_k = bars + 1, *bar_u = bars + 2, *bar_m1 = bars + 3, *bar_m2 = bars + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int v = threadIdx.x;
+  const int v = threadIdx.x & 127;          // row of S^T (TMEM lane)
+  const int wg = threadIdx.x >> 7;
   const int warp = v >> 5;
+  const bool lead = threadIdx.x == 0;
   const long long bh = blockIdx.x;
   const int n = a.n_chunks;
 
-  if (v == 0) {
+  if (lead) {
     mbar_init(bar_w, 1); mbar_init(bar_k, 1); mbar_init(bar_u, 1); mbar_init(bar_m1, 1); mbar_init(bar_m2, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmU);
   }
-  if (warp == 0) {
+  if (threadIdx.x < 32) {
     __syncwarp();
     tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
@@ -172,14 +178,14 @@ gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   uint8_t* s_a2 = smem + ScanSmem::A2;
   const long long row_base = bh * n * GC;  // first row of this sequence in the [rows, 128] tensors
 
-  if (v == 0 && n > 0) {
+  if (lead && n > 0) {
     load_tile(s_w, &tmW, bar_w, static_cast<int>(row_base));
     load_tile(s_u, &tmU, bar_u, static_cast<int>(row_base));
     load_tile(s_k, &tmK, bar_k, static_cast<int>(row_base));
   }
   // initial state: S^T[v][k] = s_init[k][v]
 #pragma unroll 1
-  for (int c0 = 0; c0 < GD; c0 += 32) {
+  for (int c0 = wg * 32; c0 < GD; c0 += 64) {
     uint32_t r[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j)
@@ -193,13 +199,13 @@ gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   for (int i = 0; i < n && ok; ++i) {
     const float eg = a.egam[bh * n + i];
     // 1. state round trip
-    state_round_trip(t_state, s_op, a.out_s + ((bh * n + i) * GD + v) * GD, eg, v);
+    state_round_trip(t_state, s_op, a.out_s + ((bh * n + i) * GD + v) * GD, eg, v, wg);
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     // 2. D1 = S^T W^T
-    if (v == 0) {
+    if (lead) {
       if (mbar_wait_bounded(bar_w, phase, abort_flag)) {
         tc_fence_after();
         issue_mma_state_times_tile(t_d1, smem_u32(s_op), smem_u32(s_w));
@@ -213,11 +219,11 @@ gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     __syncthreads();
     if (*abort_flag) { ok = false; break; }
     tc_fence_after();
-    if (v == 0 && i + 1 < n) load_tile(s_w, &tmW, bar_w, static_cast<int>(row_base + (i + 1) * GC));
+    if (lead && i + 1 < n) load_tile(s_w, &tmW, bar_w, static_cast<int>(row_base + (i + 1) * GC));
     // 3. Vn^T = U^T - D1
     __nv_bfloat16* g_v = a.out_v + (bh * n + i) * GC * GD + v;
 #pragma unroll 1
-    for (int c0 = 0; c0 < GC; c0 += 32) {
+    for (int c0 = wg * 32; c0 < GC; c0 += 64) {
       uint32_t r[32];
       tmem_ld_32x32(t_d1 + c0, r);
       tmem_ld_wait();
@@ -241,7 +247,7 @@ gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     __syncthreads();
     tc_fence_after();
     // 4. S^T += Vn^T Kd
-    if (v == 0) {
+    if (lead) {
       if (i + 1 < n) load_tile(s_u, &tmU, bar_u, static_cast<int>(row_base + (i + 1) * GC));
       if (mbar_wait_bounded(bar_k, phase, abort_flag)) {
         tc_fence_after();
@@ -255,10 +261,10 @@ gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     __syncthreads();
     if (*abort_flag) { ok = false; break; }
     tc_fence_after();
-    if (v == 0 && i + 1 < n) load_tile(s_k, &tmK, bar_k, static_cast<int>(row_base + (i + 1) * GC));
+    if (lead && i + 1 < n) load_tile(s_k, &tmK, bar_k, static_cast<int>(row_base + (i + 1) * GC));
     phase ^= 1;
   }
-  if (!ok && v == 0) {  // leave no copy in flight
+  if (!ok && lead) {  // leave no copy in flight
     int dummy = 0;
     mbar_wait_bounded(bar_w, phase, &dummy);
     mbar_wait_bounded(bar_u, phase, &dummy);
@@ -267,7 +273,7 @@ gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   // final state: s_final[k][v] = S^T[v][k]
   if (ok) {
 #pragma unroll 1
-    for (int c0 = 0; c0 < GD; c0 += 32) {
+    for (int c0 = wg * 32; c0 < GD; c0 += 64) {
       uint32_t r[32];
       tmem_ld_32x32(t_state + c0, r);
       tmem_ld_wait();
@@ -277,7 +283,7 @@ gdn_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
+  if (threadIdx.x < 32) {
     tc_fence_after();
     tmem_dealloc(*tmem_slot, 256);
   }
@@ -296,17 +302,19 @@ gdn_scan_bwd_kernel(const __grid_constant__ CUtensorMap tmKd, const __grid_const
   uint64_t *bar_a = bars, *bar_b = bars + 1, *bar_m1 = bars + 2, *bar_m2 = bars + 3;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int v = threadIdx.x;
+  const int v = threadIdx.x & 127;          // row of S^T (TMEM lane)
+  const int wg = threadIdx.x >> 7;
   const int warp = v >> 5;
+  const bool lead = threadIdx.x == 0;
   const long long bh = blockIdx.x;
   const int n = a.n_chunks;
 
-  if (v == 0) {
+  if (lead) {
     mbar_init(bar_a, 1); mbar_init(bar_b, 1); mbar_init(bar_m1, 1); mbar_init(bar_m2, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 0) {
+  if (threadIdx.x < 32) {
     __syncwarp();
     tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
@@ -348,10 +356,10 @@ gdn_scan_bwd_kernel(const __grid_constant__ CUtensorMap tmKd, const __grid_const
     tma_load_2d(s_w, &tmW, bar_b, 0, r0);
     tma_load_2d(s_w + 8192, &tmW, bar_b, 64, r0);
   };
-  if (v == 0 && n > 0) load_chunk(n - 1);
+  if (lead && n > 0) load_chunk(n - 1);
   // dS^T[v][k] = s_init[k][v]  (gradient of the final state, or zero)
 #pragma unroll 1
-  for (int c0 = 0; c0 < GD; c0 += 32) {
+  for (int c0 = wg * 32; c0 < GD; c0 += 64) {
     uint32_t r[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j)
@@ -365,13 +373,13 @@ gdn_scan_bwd_kernel(const __grid_constant__ CUtensorMap tmKd, const __grid_const
   for (int i = n - 1; i >= 0 && ok; --i) {
     const float eg = a.egam[bh * n + i];
     // 1. dS round trip: stores dS_{i+1} (the gradient of the state AFTER chunk i)
-    state_round_trip(t_state, s_op, a.out_s + ((bh * n + i) * GD + v) * GD, eg, v);
+    state_round_trip(t_state, s_op, a.out_s + ((bh * n + i) * GD + v) * GD, eg, v, wg);
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     // 2. D1 = dS^T Kd^T + dO^T P   (= dVn^T; dO^T is the dO tile read MN-major, P^T dO never leaves the SM)
-    if (v == 0) {
+    if (lead) {
       if (mbar_wait_bounded(bar_a, phase, abort_flag)) {
         tc_fence_after();
         issue_mma_state_times_tile(t_d1, smem_u32(s_op), smem_u32(s_kd));
@@ -392,7 +400,7 @@ gdn_scan_bwd_kernel(const __grid_constant__ CUtensorMap tmKd, const __grid_const
     // 3. store dVn; A2 = -dVn^T over the (now dead) Kd tile
     __nv_bfloat16* g_v = a.out_v + (bh * n + i) * GC * GD + v;
 #pragma unroll 1
-    for (int c0 = 0; c0 < GC; c0 += 32) {
+    for (int c0 = wg * 32; c0 < GC; c0 += 64) {
       uint32_t r[32];
       tmem_ld_32x32(t_d1 + c0, r);
       tmem_ld_wait();
@@ -414,7 +422,7 @@ gdn_scan_bwd_kernel(const __grid_constant__ CUtensorMap tmKd, const __grid_const
     __syncthreads();
     tc_fence_after();
     // 4. dS^T += dO^T Qd - dVn^T W
-    if (v == 0) {
+    if (lead) {
       if (mbar_wait_bounded(bar_b, phase, abort_flag)) {
         tc_fence_after();
         constexpr uint32_t idesc = umma_idesc(128, GD, 1, 1, 1);
@@ -432,17 +440,17 @@ gdn_scan_bwd_kernel(const __grid_constant__ CUtensorMap tmKd, const __grid_const
     __syncthreads();
     if (*abort_flag) { ok = false; break; }
     tc_fence_after();
-    if (v == 0 && i > 0) load_chunk(i - 1);
+    if (lead && i > 0) load_chunk(i - 1);
     phase ^= 1;
   }
-  if (!ok && v == 0) {  // leave no copy in flight
+  if (!ok && lead) {  // leave no copy in flight
     int dummy = 0;
     mbar_wait_bounded(bar_a, phase, &dummy);
     mbar_wait_bounded(bar_b, phase, &dummy);
   }
   if (ok) {
 #pragma unroll 1
-    for (int c0 = 0; c0 < GD; c0 += 32) {
+    for (int c0 = wg * 32; c0 < GD; c0 += 64) {
       uint32_t r[32];
       tmem_ld_32x32(t_state + c0, r);
       tmem_ld_wait();
@@ -452,7 +460,7 @@ gdn_scan_bwd_kernel(const __grid_constant__ CUtensorMap tmKd, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
+  if (threadIdx.x < 32) {
     tc_fence_after();
     tmem_dealloc(*tmem_slot, 256);
   }
