@@ -33,7 +33,12 @@ namespace cvb {
 
 constexpr int BC = 64;
 constexpr int BD = 128;
-constexpr int BTHREADS = 256;  // two warpgroups: warps w and w + 4 share TMEM lane quadrant w and split the columns
+// Four warpgroups: warps w, w + 4, w + 8, w + 12 share TMEM lane quadrant w and split the columns of every hand-off
+// between two MMA rounds (32 of 128, 16 of 64).  One item is a serial chain of ten such stages and its 214 KB leave room
+// for one CTA per SM, so the chain's length is the kernel's time: 16 x 1280 x 16 heads took 633 us with two warpgroups,
+// 586 with four.
+constexpr int BWG = 4;
+constexpr int BTHREADS = 128 * BWG;
 
 __device__ __forceinline__ uint32_t bsw128(uint32_t row, uint32_t chunk) {
   return row * 128u + ((chunk ^ (row & 7u)) << 4);
@@ -69,8 +74,8 @@ struct BwdSmem {
   static constexpr int SS = 180224;       // S^T: 2 x [128 x 64], later dW (16 KB; then dVb1) | Gs' | dPd'  (32 KB)
   static constexpr int DW = SS;
   static constexpr int GP = SS + 16384;
-  static constexpr int SC = 212992;       // scalars                             (6 KB)
-  static constexpr int BARS = SC + 6144;
+  static constexpr int SC = 212992;       // scalars                             (8 KB)
+  static constexpr int BARS = SC + 8192;
   static constexpr int BYTES = BARS + 256 + 1024;
 };
 
@@ -127,6 +132,11 @@ __device__ __forceinline__ void store_row32(uint8_t* tiles, int tile_stride, int
 #pragma unroll
   for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(base + bsw128(t, ch0 + j)) = pack8(f + 8 * j);
 }
+// the same for 16 elements of a [64 x 64] operand
+__device__ __forceinline__ void store_row16(uint8_t* tile, int t, int c0, const float* f) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) *reinterpret_cast<uint4*>(tile + bsw128(t, (c0 >> 3) + j)) = pack8(f + 8 * j);
+}
 __device__ __forceinline__ void store_global32(__nv_bfloat16* dst, const float* f) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(dst + 8 * j) = pack8(f + 8 * j);
@@ -150,16 +160,19 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   float* s_rk = s_c + 128;
   float* s_rq = s_c + 192;
   float* s_ec = s_c + 256;
-  float* s_rowdgg = s_c + 320;  // [2][64]: per-warpgroup partial row sums from here on
-  float* s_dba = s_c + 448;
-  float* s_dc = s_c + 576;      // [2][64]: query side, key side
-  float* s_dbv = s_c + 704;
-  float* s_dotkb = s_c + 832;
-  float* s_bk = s_c + 960;
-  float* s_aq = s_c + 1088;
+  float* s_dc = s_c + 320;      // [2][64]: query side, key side
+  float* s_rowdgg = s_c + 448;  // [BWG][64]: per-warpgroup partial row sums from here on
+  float* s_dba = s_rowdgg + BWG * 64;
+  float* s_dbv = s_dba + BWG * 64;
+  float* s_dotkb = s_dbv + BWG * 64;
+  float* s_bk = s_dotkb + BWG * 64;
+  float* s_aq = s_bk + BWG * 64;
+  auto row_total = [](const float* part, int row) {
+    return (part[row] + part[BC + row]) + (part[2 * BC + row] + part[3 * BC + row]);
+  };
 
   const int tid = threadIdx.x;
-  const int wg = tid >> 7;     // warpgroup: takes every second 32-column chunk of each stage
+  const int wg = tid >> 7;     // warpgroup: its column chunk of each stage
   const int lt = tid & 127;
   const int warp = lt >> 5;    // TMEM lane quadrant
   const bool lo = lt < BC;
@@ -211,9 +224,7 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     tmem_relinquish();
   }
   {
-    uint4* z = reinterpret_cast<uint4*>(smem + BwdSmem::Z0) + tid * 2;   // the zero tile, written once
-#pragma unroll
-    for (int j = 0; j < 2; ++j) z[j] = make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4*>(smem + BwdSmem::Z0)[tid] = make_uint4(0u, 0u, 0u, 0u);   // the zero tile, written once
   }
   BWD_PUBLISH();
   tmem_base = *tmem_slot;
@@ -239,17 +250,11 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
   {
     // T (fp32, row-major) -> bf16 tile in the 128-byte swizzle
-    const int r = tid >> 2, quarter = tid & 3;
-    const float4* src = reinterpret_cast<const float4*>(a.Tm + (item * BC + r) * BC + quarter * 16);
-    float f[16];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float4 x = src[j];
-      f[4 * j] = x.x, f[4 * j + 1] = x.y, f[4 * j + 2] = x.z, f[4 * j + 3] = x.w;
-    }
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-      *reinterpret_cast<uint4*>(smem + BwdSmem::T + bsw128(r, quarter * 2 + j)) = pack8(f + 8 * j);
+    const int r = tid >> 3, part = tid & 7;
+    const float4* src = reinterpret_cast<const float4*>(a.Tm + (item * BC + r) * BC + part * 8);
+    const float4 x0 = src[0], x1 = src[1];
+    const float f[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    *reinterpret_cast<uint4*>(smem + BwdSmem::T + bsw128(r, part)) = pack8(f);
   }
   BWD_PUBLISH();
   BWD_WAIT(bar_load, ERR_WAIT_FULL);
@@ -286,7 +291,7 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (!lo) {  // Ks_j = e^{c_j} rk_j k_j while the tensor cores run
     const float fk = s_ec[t] * s_rk[t];
 #pragma unroll 1
-    for (int c0 = wg * 32; c0 < BD; c0 += 64) {
+    for (int c0 = wg * 32; c0 < BD; c0 += 32 * BWG) {
       float f[32];
       load_row32(smem + BwdSmem::QK + 8192, 16384, t, c0, f);
 #pragma unroll
@@ -300,7 +305,7 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   {
     const float e = s_ec[t];
 #pragma unroll 1
-    for (int c0 = wg * 32; c0 < BD; c0 += 64) {
+    for (int c0 = wg * 32; c0 < BD; c0 += 32 * BWG) {
       uint32_t r[32];
       tmem_ld_32x32(tmem + TC_ACC + c0, r);
       tmem_ld_wait();
@@ -332,21 +337,21 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
   if (warp < 2) {
     const float ct = s_c[t], rqt = s_rq[t];
-#pragma unroll 1
-    for (int c0 = wg * 32; c0 < BC; c0 += 64) {
-      uint32_t r[32];
-      tmem_ld_32x32(tmem + TC_SL + c0, r);
+    {
+      const int c0 = wg * 16;
+      uint32_t r[16];
+      tmem_ld_32x16(tmem + TC_SL + c0, r);
       tmem_ld_wait();
-      float f[32];
+      float f[16];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
+      for (int j = 0; j < 16; ++j) {
         const int u = c0 + j;
         const float pd = (u <= t) ? __uint_as_float(r[j]) * __expf(ct - s_c[u]) : 0.f;
         f[j] = pd * s_rk[u];
         *reinterpret_cast<__nv_bfloat16*>(smem + BwdSmem::PT + bsw128(u, t >> 3) + (t & 7) * 2) =
             __float2bfloat16_rn(pd * rqt);
       }
-      store_row32(smem + BwdSmem::GP + 8192, 8192, t, c0, f);
+      store_row16(smem + BwdSmem::GP + 8192, t, c0, f);
     }
     fence_proxy_async_smem();
   }
@@ -358,7 +363,7 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     __nv_bfloat16* dvrow = a.dv + (row0 + t) * a.d_stride + h * BD;
     float dbv = 0.f, dot_kb = 0.f;
 #pragma unroll 1
-    for (int c0 = wg * 32; c0 < BD; c0 += 64) {
+    for (int c0 = wg * 32; c0 < BD; c0 += 32 * BWG) {
       uint32_t r[32];
       tmem_ld_32x32(tmem + TC_DX + c0, r);
       tmem_ld_wait();
@@ -376,7 +381,7 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       store_global32(dvrow + c0, f);
     }
 #pragma unroll 1
-    for (int c0 = wg * 32; c0 < BD; c0 += 64) {
+    for (int c0 = wg * 32; c0 < BD; c0 += 32 * BWG) {
       uint32_t r[32];
       tmem_ld_32x32(tmem + TC_DK + c0, r);
       tmem_ld_wait();
@@ -389,7 +394,7 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       store_row32(smem + BwdSmem::DD + 8192, 8192, t, c0, f);  // dKb k-blocks at DD + 8 KB and DD + 16 KB
     }
-    s_dbv[wg * BC + t] = dbv;      // this warpgroup's half of <dVb, v> and <dKb, k>
+    s_dbv[wg * BC + t] = dbv;      // this warpgroup's part of <dVb, v> and <dKb, k>
     s_dotkb[wg * BC + t] = dot_kb;
   }
   BWD_PUBLISH();
@@ -410,16 +415,14 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   // ---- stage 6 (lanes 64-127): M1 diag(beta) -> bf16 rows -------------------------------------------------
   if (warp >= 2) {
-#pragma unroll 1
-    for (int c0 = wg * 32; c0 < BC; c0 += 64) {
-      uint32_t r[32];
-      tmem_ld_32x32(tmem + TC_SL + c0, r);
-      tmem_ld_wait();
-      float f[32];
+    const int c0 = wg * 16;
+    uint32_t r[16];
+    tmem_ld_32x16(tmem + TC_SL + c0, r);
+    tmem_ld_wait();
+    float f[16];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(r[j]) * s_beta[c0 + j];
-      store_row32(smem + BwdSmem::M1, 8192, t, c0, f);
-    }
+    for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(r[j]) * s_beta[c0 + j];
+    store_row16(smem + BwdSmem::M1, t, c0, f);
   }
   BWD_PUBLISH();
 
@@ -446,14 +449,14 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const float ct = s_c[t], bt = s_beta[t], rkt = s_rk[t];
     float rowdgg = 0.f, dba = 0.f;
     uint8_t* gs = smem + BwdSmem::GP;
-#pragma unroll 1
-    for (int c0 = wg * 32; c0 < BC; c0 += 64) {
-      uint32_t ra[32], rg[32];
-      tmem_ld_32x32(tmem + TC_SL + c0, ra);
-      tmem_ld_32x32(tmem + TC_D1 + c0, rg);
+    {
+      const int c0 = wg * 16;
+      uint32_t ra[16], rg[16];
+      tmem_ld_32x16(tmem + TC_SL + c0, ra);
+      tmem_ld_32x16(tmem + TC_D1 + c0, rg);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
+      for (int j = 0; j < 16; ++j) {
         const int u = c0 + j;
         if (u < t) {
           const float da = -__uint_as_float(ra[j]);
@@ -495,25 +498,28 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     issue_loads(item + gridDim.x, true, false);
   }
 
-  // ---- stage 10: finish one token row per thread pair (the two warpgroups split the columns) ---------------
-  // pass 1: the row's dot product with its own (normalised) input, half per warpgroup
+  // ---- stage 10: finish one token row per four threads (the warpgroups split the columns) ---------------
+  // pass 1: the row's dot product with its own (normalised) input, a quarter per warpgroup
   if (warp < 2) {
     // key side: dK^ = ACC + e^{c_C - c_t} dKdec + beta_t e^{c_t} dKb
     const float edec = __expf(s_c[BC - 1] - s_c[t]);
     const float bek = s_beta[t] * s_ec[t];
     float bk = 0.f;
 #pragma unroll 1
-    for (int c0 = wg * 32; c0 < BD; c0 += 64) {
-      uint32_t r[32], r3[32], r7[32];
+    for (int c0 = wg * 32; c0 < BD; c0 += 32 * BWG) {
+      uint32_t r[32], r3[32];
       tmem_ld_32x32(tmem + TC_ACC + c0, r);
       tmem_ld_32x32(tmem + TC_DX + c0, r3);
-      tmem_ld_32x32(tmem + TC_DK + c0, r7);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + edec * __uint_as_float(r3[j]));
+      tmem_ld_32x32(tmem + TC_DK + c0, r3);
       tmem_ld_wait();
       float x[32];
       load_row32(smem + BwdSmem::QK + 8192, 16384, t, c0, x);
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
-        const float v = __uint_as_float(r[j]) + edec * __uint_as_float(r3[j]) + bek * __uint_as_float(r7[j]);
+        const float v = __uint_as_float(r[j]) + bek * __uint_as_float(r3[j]);
         bk += v * x[j];
         r[j] = __float_as_uint(v);
       }
@@ -525,7 +531,7 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // query side: dQ~ is complete in ACC
     float aq = 0.f;
 #pragma unroll 1
-    for (int c0 = wg * 32; c0 < BD; c0 += 64) {
+    for (int c0 = wg * 32; c0 < BD; c0 += 32 * BWG) {
       uint32_t r[32];
       tmem_ld_32x32(tmem + TC_ACC + c0, r);
       tmem_ld_wait();
@@ -540,11 +546,11 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   // pass 2: the l2-norm backward with the full dot product
   if (warp < 2) {
     const float rkt = s_rk[t];
-    const float bk = s_bk[t] + s_bk[BC + t];
+    const float bk = row_total(s_bk, t);
     const float coef = rkt * rkt * bk;
     __nv_bfloat16* dkrow = a.dk + (row0 + t) * a.d_stride + h * BD;
 #pragma unroll 1
-    for (int c0 = wg * 32; c0 < BD; c0 += 64) {
+    for (int c0 = wg * 32; c0 < BD; c0 += 32 * BWG) {
       uint32_t r[32];
       tmem_ld_32x32(tmem + TC_ACC + c0, r);
       tmem_ld_wait();
@@ -556,19 +562,19 @@ gdn_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     if (wg == 0) {
       const float bek = s_beta[t] * s_ec[t];
-      const float dot_kb = s_dotkb[t] + s_dotkb[BC + t];
-      s_dc[BC + t] = 2.f * (s_rowdgg[t] + s_rowdgg[BC + t] + bek * rkt * dot_kb) - rkt * bk;
+      const float dot_kb = row_total(s_dotkb, t);
+      s_dc[BC + t] = 2.f * (row_total(s_rowdgg, t) + bek * rkt * dot_kb) - rkt * bk;
       a.dbeta[(row0 + t) * a.H + h] =
-          s_dbv[t] + s_dbv[BC + t] + s_ec[t] * rkt * dot_kb + s_dba[t] + s_dba[BC + t];
+          row_total(s_dbv, t) + s_ec[t] * rkt * dot_kb + row_total(s_dba, t);
     }
   } else {
     const float rqt = s_rq[t];
     const float rq_ns = rqt / a.scale;
-    const float aq = s_aq[t] + s_aq[BC + t];
+    const float aq = row_total(s_aq, t);
     const float coef = rq_ns * rq_ns * aq;
     __nv_bfloat16* dqrow = a.dq + (row0 + t) * a.d_stride + h * BD;
 #pragma unroll 1
-    for (int c0 = wg * 32; c0 < BD; c0 += 64) {
+    for (int c0 = wg * 32; c0 < BD; c0 += 32 * BWG) {
       uint32_t r[32];
       tmem_ld_32x32(tmem + TC_ACC + c0, r);
       tmem_ld_wait();
