@@ -635,18 +635,31 @@ gdn_state_dot_kernel(const __nv_bfloat16* __restrict__ ST, const __nv_bfloat16* 
   float acc = 0.f;
   if (i + 1 < n) {
     const __nv_bfloat16* s = ST + (item + 1) * BD * BD;
-    for (int e = threadIdx.x * 8; e < BD * BD; e += 256 * 8) {
+    // all sixteen 16-byte loads of a thread before the first use: HBM-bound, 16 x 1280 x 16 heads 77 -> 65 us
+    uint4 xs[8], ys[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int e = (k * 256 + threadIdx.x) * 8;
+      xs[k] = *reinterpret_cast<const uint4*>(s + e);
+      ys[k] = *reinterpret_cast<const uint4*>(ds + e);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
       float x[8], y[8];
-      unpack8(*reinterpret_cast<const uint4*>(s + e), x);
-      unpack8(*reinterpret_cast<const uint4*>(ds + e), y);
+      unpack8(xs[k], x);
+      unpack8(ys[k], y);
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc += x[j] * y[j];
     }
   } else {
-    const float* s = Sf + bh * BD * BD;  // [dk][dv]: transposed against dST
-    for (int e = threadIdx.x; e < BD * BD; e += 256) {
-      const int kk = e >> 7, vv = e & 127;
-      acc += s[e] * __bfloat162float(ds[vv * BD + kk]);
+    const float* s = Sf + bh * BD * BD;  // [dk][dv]: transposed against dST; neighbouring lanes take neighbouring dv
+#pragma unroll 2
+    for (int k = 0; k < 8; ++k) {
+      const int idx = k * 256 + threadIdx.x, vv = idx & 127, kk = (idx >> 7) * 8;
+      float y[8];
+      unpack8(*reinterpret_cast<const uint4*>(ds + vv * BD + kk), y);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc += s[(kk + j) * BD + vv] * y[j];
     }
   }
   acc = warp_sum(acc);

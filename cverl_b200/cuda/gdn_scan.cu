@@ -32,7 +32,7 @@ constexpr int GD = 128;   // dk = dv
 // Two warpgroups: warps w and w + 4 share TMEM lane quadrant w (the same 32 rows of the state) and take every second
 // 32-column chunk of each TMEM -> register pass.  The scan is one serial chain per sequence, and those passes are its
 // longest links: 16 sequences of 1280 x 16 heads took 133 us forward and 135 us backward with one warpgroup,
-// 121 and 131 us with two (what is left is mostly the MMA and barrier latency of 20 chunks in a row).
+// 120 and 131 - 135 us with two (what is left is mostly the MMA and barrier latency of 20 chunks in a row).
 constexpr int GTHREADS = 256;
 
 // byte offset of 16-byte chunk `chunk` of row `row` in a 128-byte-swizzled tile with 128-byte rows
