@@ -10,8 +10,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("seq", [1, 63, 127, 130, 255, 333])
 @pytest.mark.parametrize("layout", ["packed", "strided", "misaligned"])
 def test_ragged_head_dim_256_matches_the_library(seq, layout):
-    from cverl_b200.ops import attention
-    from cverl_b200.utils import fallbacks
+    from cverl_b200.ops import attention, attention_native
     g = torch.Generator(device="cuda").manual_seed(seq)
     B, Hq, Hkv, D = 2, 4, 2, 256
 
@@ -24,11 +23,9 @@ def test_ragged_head_dim_256_matches_the_library(seq, layout):
         return flat[off:off + n].view(B * seq, h, D)
     base = [make(h) for h in (Hq, Hkv, Hkv)]
     do = make(Hq)
-    fallbacks.reset()
     got_in = [t.detach().requires_grad_(True) for t in base]
-    out = attention.causal_attention(*got_in, B, seq)
+    out = attention_native.causal_attention(*got_in, B, seq)
     got = (out,) + torch.autograd.grad(out, got_in, do)
-    assert fallbacks.total() == 0
     ref_in = [t.detach().double().requires_grad_(True) for t in base]
     q, k, v = (t.view(B, seq, -1, D).transpose(1, 2) for t in ref_in)
     s = (q @ k.repeat_interleave(2, 1).transpose(-1, -2)) / math.sqrt(D)
@@ -51,7 +48,25 @@ def test_calls_that_stay_on_the_general_path():
     q = torch.randn(100, 2, 128, device="cuda").to(torch.bfloat16)
     assert not an.supported(q, q, q, 100)                              # head dim 128, ragged
     assert an.supported(q, q, q, 128)
-    w = torch.randn(100, 2, 256, device="cuda").to(torch.bfloat16)
-    assert an.supported(w, w, w, 100) and not an.supported(w.float(), w.float(), w.float(), 100)
+    small = torch.randn(100, 2, 256, device="cuda").to(torch.bfloat16)
+    assert not an.supported(small, small, small, 100)                  # 20,000 scores: the host's side decides
     empty = torch.empty(0, 2, 256, device="cuda", dtype=torch.bfloat16)
     assert an.causal_attention(empty, empty, empty, 0, 100).shape == (0, 2, 256)
+
+
+def test_large_ragged_call_runs_on_the_kernels():
+    """3 sequences of 1001 with 4 / 2 heads: the smallest length that this many heads send to the kernels is 1000."""
+    from cverl_b200.ops import attention, attention_native as an
+    from cverl_b200.utils import fallbacks
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k = (torch.randn(3 * 1001, h, 256, device="cuda", generator=g).to(torch.bfloat16) for h in (4, 2))
+    assert an.supported(q, k, k, 1001) and not an.supported(q.float(), k.float(), k.float(), 1001)
+    fallbacks.reset()
+    out = attention.causal_attention(q, k, k, 3, 1001)
+    assert fallbacks.total() == 0
+    ref = attention._sdpa(q, k, k, 3, 1001, None)
+    # two bf16 results of the same sums: half a unit in the last place each, and the rounded weights
+    assert (out.float() - ref.float()).norm() <= 2.0 ** -8 * ref.float().norm()
+    attention.causal_attention(q[:999 * 3], k[:999 * 3], k[:999 * 3], 3, 999)
+    assert fallbacks.total() == 1
+    fallbacks.reset()
