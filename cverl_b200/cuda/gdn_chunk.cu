@@ -117,16 +117,23 @@ gdn_chunk_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
-  if (warp == 0) {  // inclusive scan of g, two neighbouring tokens per lane
-    const float g0 = s_c[2 * tid], g1 = s_c[2 * tid + 1];
-    float incl = g0 + g1;
+  if (tid == 0) {
+    // Inclusive scan of g, in token order: a prefix holds nothing of a later gate, and prefixes of gates <= 0 never rise
+    // (taking one back out of a longer sum leaves the rounding error of that sum, which a strong decay makes large).
+    // The 63 dependent additions run out of registers while Q, K and V are on their way.
+    float4* c4 = reinterpret_cast<float4*>(s_c);
+    float4 x[CC / 4];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float up = __shfl_up_sync(0xffffffffu, incl, o);
-      if (tid >= o) incl += up;
+    for (int i = 0; i < CC / 4; ++i) x[i] = c4[i];
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < CC / 4; ++i) {
+      x[i].x = acc += x[i].x;
+      x[i].y = acc += x[i].y;
+      x[i].z = acc += x[i].z;
+      x[i].w = acc += x[i].w;
+      c4[i] = x[i];
     }
-    s_c[2 * tid] = incl - g1;
-    s_c[2 * tid + 1] = incl;
   }
   bool ok = mbar_wait_bounded(bar_load, 0, abort_flag);
   if (!ok) {
