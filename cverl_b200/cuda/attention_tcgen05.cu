@@ -11,19 +11,15 @@
 // NT = 1 the slots alternate by key block (S of block j + 1 is issued before O += P V of block j), at NT = 2 each
 // tile has its own.  MMAs of one CTA retire in issue order, so a slot is overwritten by the next S only after its P
 // has been read, without a wait.
-// O is rescaled only when a row's maximum has grown past a bound since the last rescale (the sums use the same stale
-// maximum): 2^8 with the plain sum of the weights where the lengths are multiples of 128.  Other lengths (head dim 256)
-// have the library's kernel as their alternative and match its error: bound 2^2, since the weight of the largest score
-// is exact only while its maximum is, and O divided by the sum of the ROUNDED weights, which takes the common part of
-// their rounding errors out of the result (LSE keeps the plain sum).  Error of the bf16 output against 64 bits,
-// 24 x 333 / 4 x 1500: library 1.945e-3 / 2.011e-3, this 1.944e-3 / 2.027e-3, the faster form 1.968e-3 / 2.056e-3; dK and dV
-// are closer than the library's by a fifth either way.  It costs 15 % of the forward pass (16 x 1280: 167 us).
+// The accumulator O is rescaled only when a row's maximum has grown by more than 2^8 since the last rescale (the
+// stale maximum keeps P <= 256, exactness is kept because l uses the same maximum).
 // Query / key position offsets make the same kernel serve the hops of context-parallel ring attention: it returns the
 // un-merged (O, LSE) of one key range.  Sequences of any length: rows past the end are zero-filled by TMA, masked as
 // keys and clipped by the TMA store as queries.
 // Bound by the tensor cores at head dim 256 and by the exponentials at 128.
-// Causal, 16 x 1280 with 8 query and 2 kv heads of 256: 150 us (709 TFLOP/s), 269 us as one serial chain per CTA in blocks of
-// 64 keys.  1 x 8192 of the same heads runs at 1,276 TFLOP/s, 2 x 4096 with 32 heads of 128 at 904; at 1280 what remains is the fill and drain of each CTA's chain of 5.5 blocks on average.
+// Causal, 16 x 1280 with 8 query and 2 kv heads of 256: 143 - 150 us (709 - 744 TFLOP/s), 269 us as one serial chain
+// per CTA in blocks of 64 keys.  1 x 8192 of the same heads runs at 1,276 TFLOP/s, 2 x 4096 with 32 heads of 128 at 904; at
+// 1280 what remains is the fill and drain of each CTA's chain of 5.5 blocks on average.
 //
 // The reference calls at::scaled_dot_product_attention (src/model/qwen3_5_text.cc:1068-1075) and, for
 // context parallelism, a scalar SIMT kernel (cuda/cp_attention_cuda.cu).
@@ -63,14 +59,14 @@ __device__ __forceinline__ uint32_t asw128(uint32_t row, uint32_t chunk) {
   return row * 128u + ((chunk ^ (row & 7u)) << 4);
 }
 
-template <int D, bool ROUNDED_SUM>
+template <int D>
 __global__ void __launch_bounds__(AttCfg<D>::THREADS, 1)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                      const AttArgs a) {
   using C = AttCfg<D>;
   constexpr int NT = C::NT, PER = C::PER, NB = D / 64;
-  constexpr float GROW = ROUNDED_SUM ? 2.f : 8.f;   // log2 of the growth that O tolerates without a rescale
+  constexpr float GROW = 8.f;   // log2 of the growth that O tolerates without a rescale
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::BARS);
@@ -301,8 +297,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const long long qpos = a.q_pos0 + qi;
     const long long first_pos = a.q_pos0 + q0 + t * AT_BQ;
     const int nt = t == 0 ? n[0] : n[NT - 1];
-    // m_used: the maximum that O and the sums refer to; l, l_r: sums of the weights and of the rounded weights
-    float m_used = -INFINITY, l = 0.f, l_r = 0.f;
+    float m_used = -INFINITY, l = 0.f;   // the maximum that O and l refer to; sum of the weights
     bool ok = true;
     auto wait = [&](uint64_t* bar, uint32_t par) {
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, par, abort_flag));
@@ -346,25 +341,22 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         alpha = m_used == -INFINITY ? 0.f : exp2f(m_used - m_new);
         m_used = m_new;
         l *= alpha;
-        l_r *= alpha;
       }
       const float mm = m_used == -INFINITY ? 0.f : m_used;
-      float sum[4], sum_r[4];
+      float sum[4];
       uint32_t p[4][16];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        sum[c] = sum_r[c] = 0.f;
+        sum[c] = 0.f;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const float p0 = exp2f(__uint_as_float(r[c][2 * i]) * a.scale_log2 - mm);
           const float p1 = exp2f(__uint_as_float(r[c][2 * i + 1]) * a.scale_log2 - mm);
           sum[c] += p0 + p1;
           p[c][i] = pack_bf16x2(p0, p1);
-          if (ROUNDED_SUM) sum_r[c] += __uint_as_float(p[c][i] << 16) + __uint_as_float(p[c][i] & 0xffff0000u);
         }
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
-      if (ROUNDED_SUM) l_r += (sum_r[0] + sum_r[1]) + (sum_r[2] + sum_r[3]);
       if (grow && j > 0) {
         // O must hold the blocks before.  At NT = 2 that is so once S of this block is complete, at NT = 1 once S of the
         // next one is (both were issued after O += P V of block j - 1, and a commit covers all MMAs issued before it);
@@ -395,8 +387,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     if (ok && q0 + t * AT_BQ < a.Sq) {
       tc_fence_after();
       // O / l as bf16 over this tile's Q (its last S is complete), then out by TMA, which drops rows past the end
-      const float total = ROUNDED_SUM ? l_r : l;
-      const float inv = total > 0.f ? 1.f / total : 0.f;
+      const float inv = l > 0.f ? 1.f / l : 0.f;
       uint8_t* stage = smem + C::Q + t * (D * 256);
 #pragma unroll 1
       for (int c0 = 0; c0 < D; c0 += 32) {
@@ -442,7 +433,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
 }
 
-template <int D, bool ROUNDED_SUM>
+template <int D>
 static int launch_fwd(const void* q, const void* k, const void* v, void* out, float* lse, long long B, int Sq,
                       int Skv, int Hq, int Hkv, float scale, int causal, long long q_pos0, long long k_pos0,
                       int* status, cudaStream_t st) {
@@ -461,14 +452,14 @@ static int launch_fwd(const void* q, const void* k, const void* v, void* out, fl
   a.status = status;
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(attention_fwd_kernel<D, ROUNDED_SUM>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::BYTES) !=
+    if (cudaFuncSetAttribute(attention_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::BYTES) !=
         cudaSuccess)
       return -11;
     attr = true;
   }
   const long long blocks = static_cast<long long>((Sq + C::NT * AT_BQ - 1) / (C::NT * AT_BQ)) * Hq * B;
   if (blocks > 0x7fffffffLL) return -2;
-  attention_fwd_kernel<D, ROUNDED_SUM><<<static_cast<unsigned>(blocks), C::THREADS, C::BYTES, st>>>(mq, mk, mv, mo, a);
+  attention_fwd_kernel<D><<<static_cast<unsigned>(blocks), C::THREADS, C::BYTES, st>>>(mq, mk, mv, mo, a);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -489,8 +480,7 @@ extern "C" int cvb_attention_fwd(const void* q, const void* k, const void* v, vo
     if (reinterpret_cast<uintptr_t>(p) & 15) return -3;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (D != 128 && D != 256) return -1;
-  auto launch = D == 128 ? launch_fwd<128, false>
-                         : (Sq % 128 || Skv % 128 ? launch_fwd<256, true> : launch_fwd<256, false>);
+  auto launch = D == 128 ? launch_fwd<128> : launch_fwd<256>;
   return launch(q, k, v, out, lse, B, Sq, Skv, Hq, Hkv, scale, causal, q_pos0, k_pos0, status, st);
 }
 

@@ -49,10 +49,10 @@ def causal_attention(q, k, v, batch: int, seq: int, scale: float | None = None):
         backend = os.environ.get("CVERL_B200_ATTENTION", "auto")
         if backend != "sdpa":
             from . import attention_native
-            if attention_native.supported(q, k, v, seq) and (seq % 128 == 0 or scale is None or scale > 0):
+            if attention_native.supported(q, k, v, seq):
                 return attention_native.causal_attention(q, k, v, batch, seq, scale)
             from ..utils import fallbacks
             fallbacks.note("causal_attention", f"dtype {q.dtype}, head dim {q.shape[-1]}, sequence length {seq}: the "
-                                               f"tcgen05 kernels take bf16, head dim 128 / 256, length % 128 == 0 (or large calls of 256)")
+                                               f"tcgen05 kernels take bf16, head dim 128 / 256, length % 128 == 0")
         return _sdpa(q, k, v, batch, seq, scale)
     return causal_attention_ref(q, k, v, batch, seq, scale)

@@ -20,25 +20,19 @@ def _enabled() -> bool:
     return os.environ.get("CVERL_B200_ATTENTION", "auto") in ("auto", "native")
 
 
-# scores (sequences x query heads x length^2) of a ragged call from which on the kernels are the faster side
-_RAGGED_MIN_SCORES = 12_000_000
-
-
 def supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, seq: int) -> bool:
-    """bf16, head dim 128 / 256, sequence length a multiple of 128; at head dim 256 also other lengths, unless the call
-    is small.
+    """bf16, head dim 128 or 256, sequence length a multiple of 128.
 
-    The kernels take any length at both head dims.  Where a length is no multiple of 128 the library is the faster side
-    at head dim 128 (forward and backward of 4 x 1500, 32 / 4 heads: 430 us against about 660 for 4 x 1536 here); at 256 it
-    is not (8 x 1088, 8 / 2 heads: 601 us in the library, 416 here; 24 x 333 forward: 69.7 against 47.2) until the host's
-    side of the calls is the time: 4 x 391 (4.9 M scores) and 34 x 88 (2.1 M), forward and backward, 176 and 173 us a pass
-    in the library, 199 and 197 here."""
+    The kernels take any length, but no rule on the length alone makes them the faster side at the others, and a rule on the
+    batch as well would give a sequence other roundings in a small batch than in a large one (old log-probabilities scored
+    at one micro-batch size, new ones formed at another).  8 / 2 heads of 256, forward and backward: 8 x 1088 704 us in the
+    library and 419 here, but 1 x 1225 200 and 333, 1 x 2500 545 and 633, since a key block's CTA walks the queries of a
+    whole GQA group; head dim 128, 32 / 4 heads: 4 x 1500 467 in the library, 4 x 1536 660 here."""
     if not (_enabled() and q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16):
         return False
     d = q.shape[-1]
-    if not (d in (128, 256) and v.shape[-1] == d and k.shape[-1] == d and q.shape[-2] % k.shape[-2] == 0):
-        return False
-    return seq % 128 == 0 or (d == 256 and q.numel() // d * seq >= _RAGGED_MIN_SCORES)
+    return d in (128, 256) and v.shape[-1] == d and k.shape[-1] == d and seq % 128 == 0 and \
+        q.shape[-2] % k.shape[-2] == 0
 
 
 def _operand(t: torch.Tensor) -> torch.Tensor:

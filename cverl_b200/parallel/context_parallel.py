@@ -113,8 +113,7 @@ def _native_hops(q, k, v, shard_len: int, original_len: int, cp: int) -> bool:
     if not q.is_cuda:
         return False
     from ..ops import attention_native
-    return (shard_len % 128 == 0 and attention_native.supported(q, k, v, shard_len)
-            and original_len == cp * shard_len and q.shape[2] == shard_len)
+    return attention_native.supported(q, k, v, shard_len) and original_len == cp * shard_len and q.shape[2] == shard_len
 
 
 def _ring_forward_native(ctx, q, k, v, group, cp_rank, cp, shard_len, original_len, scale):

@@ -1,4 +1,5 @@
-"""Which calls of ``causal_attention`` run on the kernels, and that ragged ones give what the general path gives."""
+"""Which calls of ``causal_attention`` run on the kernels, and that the kernels give at ragged lengths what the general
+path gives."""
 import math
 
 import pytest
@@ -43,30 +44,40 @@ def test_ragged_head_dim_256_matches_the_library(seq, layout):
         assert err <= 4 * 2.0 ** -9 * r.norm() or err <= 2 * other + 1e-9, (float(err), float(other))
 
 
-def test_calls_that_stay_on_the_general_path():
-    from cverl_b200.ops import attention_native as an
-    q = torch.randn(100, 2, 128, device="cuda").to(torch.bfloat16)
-    assert not an.supported(q, q, q, 100)                              # head dim 128, ragged
-    assert an.supported(q, q, q, 128)
-    small = torch.randn(100, 2, 256, device="cuda").to(torch.bfloat16)
-    assert not an.supported(small, small, small, 100)                  # 20,000 scores: the host's side decides
-    empty = torch.empty(0, 2, 256, device="cuda", dtype=torch.bfloat16)
-    assert an.causal_attention(empty, empty, empty, 0, 100).shape == (0, 2, 256)
+def _qk(batch, seq, d=256, hq=4, hkv=2, seed=5):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return [torch.randn(batch * seq, h, d, device="cuda", generator=g).to(torch.bfloat16) for h in (hq, hkv)]
 
 
-def test_large_ragged_call_runs_on_the_kernels():
-    """3 sequences of 1001 with 4 / 2 heads: the smallest length that this many heads send to the kernels is 1000."""
+@pytest.mark.parametrize("d", [128, 256])
+@pytest.mark.parametrize("seq", [100, 128, 1001, 1024])
+def test_the_route_depends_on_the_length_alone(d, seq):
+    """A sequence takes the same path, and with it the same roundings, in a small batch and in a large one."""
     from cverl_b200.ops import attention, attention_native as an
     from cverl_b200.utils import fallbacks
-    g = torch.Generator(device="cuda").manual_seed(5)
-    q, k = (torch.randn(3 * 1001, h, 256, device="cuda", generator=g).to(torch.bfloat16) for h in (4, 2))
-    assert an.supported(q, k, k, 1001) and not an.supported(q.float(), k.float(), k.float(), 1001)
+    for batch in (1, 3, 40):
+        q, k = _qk(batch, seq, d)
+        assert an.supported(q, k, k, seq) == (seq % 128 == 0)
+        fallbacks.reset()
+        attention.causal_attention(q, k, k, batch, seq)
+        assert fallbacks.total() == (seq % 128 != 0)
+    assert not an.supported(q.float(), k.float(), k.float(), seq)
+    empty = torch.empty(0, 2, d, device="cuda", dtype=torch.bfloat16)
+    assert an.causal_attention(empty, empty, empty, 0, 100).shape == (0, 2, d)
     fallbacks.reset()
-    out = attention.causal_attention(q, k, k, 3, 1001)
-    assert fallbacks.total() == 0
-    ref = attention._sdpa(q, k, k, 3, 1001, None)
-    # two bf16 results of the same sums: half a unit in the last place each, and the rounded weights
-    assert (out.float() - ref.float()).norm() <= 2.0 ** -8 * ref.float().norm()
-    attention.causal_attention(q[:999 * 3], k[:999 * 3], k[:999 * 3], 3, 999)
-    assert fallbacks.total() == 1
-    fallbacks.reset()
+
+
+def test_ragged_calls_keep_the_transforms_of_the_general_path():
+    """Function transforms run, a second derivative is refused instead of left out."""
+    from cverl_b200.ops import attention
+    (q, k), seq = _qk(3, 1001), 1001
+    one = attention.causal_attention(q, k, k, 3, seq)
+    two = torch.func.vmap(lambda a, b: attention.causal_attention(a, b, b, 3, seq))(torch.stack([q, q]), torch.stack([k, k]))
+    # bf16 results of the same sums, in another order if the library splits the larger batch differently
+    assert (two.float() - one.float()).norm() <= 2 ** 0.5 * 2.0 ** -8 * one.float().norm()
+    dq = torch.func.grad(lambda a: attention.causal_attention(a, k, k, 3, seq).float().sum())(q)
+    a = q.detach().requires_grad_(True)
+    (want,) = torch.autograd.grad(attention.causal_attention(a, k, k, 3, seq).float().sum(), a, create_graph=True)
+    assert (dq.float() - want.float()).norm() <= 2.0 ** -8 * want.detach().float().norm()
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(want.float().pow(2).sum(), a)
