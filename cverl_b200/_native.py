@@ -73,6 +73,7 @@ _CUDA_PROTOS = {
     "cvb_masked_whiten": "pp l i pp p",
     "cvb_kl_penalty": "ppp l ii p",
     "cvb_gae": "pppppp l i ff p p",
+    "cvb_rl_one_launch_limits": "pp",
     "cvb_grpo_advantage": "ppp f i ppp l i p",
     "cvb_ppo_loss": "pppppppp l i ffff i f i f p p",
     "cvb_sumsq_f32": "p l f p p",

@@ -445,6 +445,13 @@ extern "C" int cvb_gae(const float* rew, const float* val, const float* mask, fl
       rew, val, mask, adv_raw, ret, rows, cols, gamma, lam);
   return cvb_masked_whiten(adv_raw, mask, rows * cols, 1, adv_out, ws, stream);
 }
+// The limits up to which a call is one launch (three otherwise), for whoever counts launches.
+extern "C" int cvb_rl_one_launch_limits(long long* tokens, long long* advantage_rows) {
+  *tokens = RL_SMALL_N;
+  *advantage_rows = RL_SMALL_ROWS;
+  return 0;
+}
+
 extern "C" int cvb_grpo_advantage(const float* rewards, const float* mask, const long long* gid, float eps,
                                   int norm_by_std, float* adv, float* ret, float* row_scratch, long long rows,
                                   int cols, void* stream) {

@@ -14,6 +14,7 @@ Three interchangeable implementations of one contract
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from dataclasses import dataclass
 
 from typing import Optional
@@ -308,6 +309,14 @@ def fused_gae(token_level_rewards, values, response_mask, gamma: float, lam: flo
     return adv, ret
 
 
+@functools.lru_cache(maxsize=1)
+def _one_launch_limits():
+    """(tokens, advantage rows) up to which the loss and the advantage are one launch each; three above."""
+    tokens, rows = C.c_longlong(), C.c_longlong()
+    nv.check(nv.cuda().cvb_rl_one_launch_limits(C.addressof(tokens), C.addressof(rows)), "cvb_rl_one_launch_limits")
+    return tokens.value, rows.value
+
+
 def fused_grpo_advantage(token_level_rewards, response_mask, group_ids, epsilon: float = 1e-6,
                          norm_adv_by_std: bool = True):
     rew, msk = _f32c(token_level_rewards), _f32c(response_mask)
@@ -318,7 +327,8 @@ def fused_grpo_advantage(token_level_rewards, response_mask, group_ids, epsilon:
     nv.check(nv.cuda().cvb_grpo_advantage(rew.data_ptr(), msk.data_ptr(), gid.data_ptr(), epsilon,
                                           int(norm_adv_by_std), adv.data_ptr(), None, scratch.data_ptr(), rows,
                                           cols, nv.stream()), "cvb_grpo_advantage")
-    count_launch(3)
+    tokens, small_rows = _one_launch_limits()
+    count_launch(1 if rows * cols <= tokens and rows <= small_rows else 3)
     return adv, adv
 
 
@@ -343,7 +353,7 @@ def fused_ppo_loss(old_log_prob, log_prob, advantages, response_mask, ref_log_pr
                                     clip_ratio_low, clip_ratio_high, clip_ratio_c, agg_mode(agg), kl_coef,
                                     kl_kind(kl_penalty_kind), loss_scale, _workspace(lp.device).data_ptr(),
                                     nv.stream()), "cvb_ppo_loss")
-    count_launch(3)
+    count_launch(1 if rows * cols <= _one_launch_limits()[0] else 3)
     return metrics, grad
 
 
