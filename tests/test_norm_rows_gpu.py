@@ -18,8 +18,14 @@ def _close(a, r, tol):
     assert (a.double() - r).norm() <= tol * r.norm() + 1e-6, float((a.double() - r).norm() / r.norm())
 
 
-@pytest.mark.parametrize("D", [64, 128, 256, 512, 768, 1024, 1280])
-@pytest.mark.parametrize("rows", [1, 3, 9, 70, 1000])
+def _shapes(small, above):
+    """Every small shape, and the shapes above one resident wave (148 SMs x 2 - 3 blocks of 8 warps), whose warps walk
+    several row groups, the last one with a remainder."""
+    return [s for group in small for s in group] + above
+
+
+@pytest.mark.parametrize("D,rows", _shapes([[(D, r) for r in (1, 3, 9, 70, 1000)] for D in (64, 128, 256, 512, 768, 1024, 1280)],
+                                           [(64, 120_003), (256, 40_961), (768, 9_001), (1024, 9_001), (1024, 40_961)]))
 @pytest.mark.parametrize("resid", [False, True])
 def test_add_rmsnorm_backward(D, rows, resid):
     from cverl_b200 import ops
@@ -37,8 +43,9 @@ def test_add_rmsnorm_backward(D, rows, resid):
     _close(w.main_grad, dw, DW_TOL)
 
 
-@pytest.mark.parametrize("D", [64, 128, 256])
-@pytest.mark.parametrize("tokens,heads", [(1, 1), (5, 3), (67, 16)])
+@pytest.mark.parametrize("D,tokens,heads", _shapes([[(D, *s) for s in ((1, 1), (5, 3), (67, 16))]
+                                                    for D in (64, 128, 256, 512, 768, 1024)],
+                                                   [(128, 6_667, 3), (256, 2_501, 4), (768, 3_001, 3), (1024, 3_001, 3)]))
 def test_gated_rmsnorm_backward(D, tokens, heads):
     from cverl_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(D + tokens)
@@ -53,8 +60,9 @@ def test_gated_rmsnorm_backward(D, tokens, heads):
         _close(a, r, DX_TOL)
 
 
-@pytest.mark.parametrize("D,rot", [(64, 16), (128, 128), (256, 64)])
-@pytest.mark.parametrize("tokens,heads", [(1, 1), (3, 5), (130, 8)])
+@pytest.mark.parametrize("D,rot,tokens,heads", _shapes([[(*d, *s) for s in ((1, 1), (3, 5), (130, 8))]
+                                                        for d in ((64, 16), (128, 128), (256, 64))],
+                                                       [(64, 16, 13_337, 9), (128, 128, 6_667, 6), (256, 64, 6_667, 3)]))
 @pytest.mark.parametrize("use_norm", [True, False])
 def test_headnorm_rope_backward(D, rot, tokens, heads, use_norm):
     from cverl_b200 import ops
