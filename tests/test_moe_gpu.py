@@ -53,3 +53,33 @@ def test_expert_block_matches_a_loop_over_experts(T, E, k, H, inter, one, main_g
         # a routing weight's gradient is <dy, y> and may cancel: its error is relative to |dy| |y|, not to the result
         size = (dy.float().norm(dim=-1, keepdim=True) * norms).norm() if r is ref[1] else r.grad.norm()
         assert (ga.float() - r.grad).norm() <= tol * size + 1e-6 * r.grad.numel() ** 0.5
+
+
+@pytest.mark.parametrize("layout", ["strided", "misaligned"])
+def test_expert_block_copies_rows_that_cannot_be_read_in_place(layout):
+    """Token rows and output gradients with a row stride, or 2 bytes off a 16-byte boundary, give what packed ones give."""
+    from cverl_b200 import _native as nv
+    from cverl_b200.ops.moe import moe_experts, supported
+    g = torch.Generator(device="cuda").manual_seed(3)
+    T, E, k, H, inter = 130, 4, 2, 136, 64
+
+    def bf(*s, scale=1.0):
+        return (scale * torch.randn(*s, device="cuda", generator=g)).to(torch.bfloat16)
+
+    def odd(t):
+        if layout == "strided":
+            return torch.stack([t, t], 1)[:, 0]
+        buf = torch.empty(t.numel() + 8, device="cuda", dtype=t.dtype)
+        return buf[1:1 + t.numel()].view(t.shape).copy_(t)
+    x, dy, gu, dn = bf(T, H), bf(T, H), bf(E, 2 * inter, H, scale=H ** -0.5), bf(E, H, inter, scale=inter ** -0.5)
+    ids = torch.rand(T, E, device="cuda", generator=g).topk(k, -1).indices
+    w = torch.softmax(torch.randn(T, k, device="cuda", generator=g), -1)
+    res = []
+    for make in (lambda t: t, odd):
+        a, b = make(x).detach().requires_grad_(True), w.clone().requires_grad_(True)
+        assert supported(a, gu, dn, k)
+        y = moe_experts(a, ids, b, gu, dn)
+        res.append((y.detach(),) + torch.autograd.grad(y, (a, b), make(dy)))
+    nv.check_status()
+    for p, q in zip(*res):
+        assert torch.equal(p, q)
