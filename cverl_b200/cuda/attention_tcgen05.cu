@@ -17,9 +17,11 @@
 // un-merged (O, LSE) of one key range.  Sequences of any length: rows past the end are zero-filled by TMA, masked as
 // keys and clipped by the TMA store as queries.
 // Bound by the tensor cores at head dim 256 and by the exponentials at 128.
-// Causal, 16 x 1280 with 8 query and 2 kv heads of 256: 143 - 150 us (709 - 744 TFLOP/s), 269 us as one serial chain
-// per CTA in blocks of 64 keys.  1 x 8192 of the same heads runs at 1,276 TFLOP/s, 2 x 4096 with 32 heads of 128 at 904; at
-// 1280 what remains is the fill and drain of each CTA's chain of 5.5 blocks on average.
+// Causal, 16 x 1280 with 8 query and 2 kv heads of 256: 146 us (738 TFLOP/s), 269 us as one serial chain per CTA in
+// blocks of 64 keys.  1 x 8192 of the same heads runs at 1,270 TFLOP/s, 2 x 4096 with 32 heads of 128 at 912; at 1280
+// what remains is the fill and drain of each CTA's chain of 5.5 blocks on average.
+// A key that a query must not see has the weight 0 in P, and 0 times a value that is not finite is NaN: such a value
+// reaches every query of the tile of 128 that its key lies in, earlier ones among them.
 //
 // The reference calls at::scaled_dot_product_attention (src/model/qwen3_5_text.cc:1068-1075) and, for
 // context parallelism, a scalar SIMT kernel (cuda/cp_attention_cuda.cu).
@@ -358,9 +360,9 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       if (grow && j > 0) {
-        // O must hold the blocks before.  At NT = 2 that is so once S of this block is complete, at NT = 1 once S of the
-        // next one is (both were issued after O += P V of block j - 1, and a commit covers all MMAs issued before it);
-        // before the last block there is a barrier of its own.
+        // O must hold the blocks before.  At NT = 2 that is so once S of this block is complete, at NT = 1 once S of
+        // the next one is (both were issued after O += P V of block j - 1, and a commit covers all MMAs issued before
+        // it); before the last block there is a barrier of its own.
         if (NT == 1) {
           if (j + 1 < nt ? !wait(&bar_s[slot ^ 1], ((j + 1) >> 1) & 1) : !wait(bar_pen, 0)) break;
           tc_fence_after();
@@ -507,7 +509,7 @@ extern "C" int cvb_attention_fwd(const void* q, const void* k, const void* v, vo
 // the warps fetch S, dP of j + 1.
 // Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 two warpgroups that split the 64 columns of a step.
 // A CTA of BWD_K / BWD_V / BWD_KV walks the queries of EVERY head of its GQA group, so dK / dV come out summed.
-// Causal, 16 x 1280 with 8 query and 2 kv heads of 256: dQ 230, dK 207, dV 143 and Delta 37 us; one serial chain of MMA
+// Causal, 16 x 1280 with 8 query and 2 kv heads of 256: dQ 232, dK 209, dV 145 and Delta 31 us; one serial chain of MMA
 // and softmax per CTA in two kernels, with dQ reduced into a cleared fp32 buffer and transposed, took 1,130.  A step of
 // 64 columns of BWD_K takes about 1.9 us: three MMA units against 64 KB of operands, as many bytes per unit as the
 // forward reads.
@@ -876,9 +878,11 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_cons
       for (int c = 0; c < 4; ++c) {
         const uint32_t off = asw128(row, wg * 4 + c);
         if (C::ACC_V)
-          *reinterpret_cast<uint4*>(smem + C::PT + off) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+          *reinterpret_cast<uint4*>(smem + C::PT + off) =
+              make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
         if (C::ACC_1)
-          *reinterpret_cast<uint4*>(smem + C::DS + off) = make_uint4(dk[4 * c], dk[4 * c + 1], dk[4 * c + 2], dk[4 * c + 3]);
+          *reinterpret_cast<uint4*>(smem + C::DS + off) =
+              make_uint4(dk[4 * c], dk[4 * c + 1], dk[4 * c + 2], dk[4 * c + 3]);
       }
       fence_proxy_async_smem();
       __syncwarp();
@@ -938,12 +942,14 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmA1, const __grid_cons
 }
 
 // delta[b, h, q] = sum_d dO[b, q, h, d] * O[b, q, h, d]     (a warp takes DELTA_ROWS (token, head) rows of up to 256)
-// HBM-bound; with one row per warp the index arithmetic of the store was as long as the row (16 x 1280 x 8 of 256: 37 -> 31 us)
+// HBM-bound; with one row per warp the index arithmetic of the store was as long as the row (16 x 1280 x 8 of 256:
+// 37 -> 31 us)
 constexpr int DELTA_ROWS = 4;
 __global__ void __launch_bounds__(256)
 attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                        float* __restrict__ delta, long long rows, int Sq, int Hq, int D) {
-  const long long row0 = ((static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) >> 5) * DELTA_ROWS;   // (b*Sq + q)*Hq + h
+  // rows are (b * Sq + q) * Hq + h
+  const long long row0 = ((static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) >> 5) * DELTA_ROWS;
   const int lane = threadIdx.x & 31;
   const int c = lane * 8;
   uint4 a[DELTA_ROWS], g[DELTA_ROWS];

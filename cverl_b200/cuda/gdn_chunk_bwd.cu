@@ -19,9 +19,9 @@
 // gdn_state_dot.  Every product runs as M = 128 tcgen05 MMAs: two 64-row operands are stacked
 // ([Q;K], [dVn;dO], [Gs';dPd']) or the unused half reads don't-care rows (a zero tile where the
 // accumulator is shared).  TMEM lanes 0-63 carry the key-side results, lanes 64-127 the query-side
-// and 64 x 64 ones.  The CTA has two warpgroups: warps w and w + 4 may both read TMEM lane quadrant w, so
-// every TMEM -> registers -> shared-memory hand-off between two MMA rounds is split by columns (each
-// warpgroup takes every second 32-column chunk), and a token row's scalar results are the sum of two
+// and 64 x 64 ones.  The CTA has four warpgroups: warps w, w + 4, w + 8 and w + 12 may all read TMEM lane
+// quadrant w, so every TMEM -> registers -> shared-memory hand-off between two MMA rounds is split by
+// columns (a warpgroup takes 32 of 128 or 16 of 64), and a token row's scalar results are the sum of four
 // partial sums exchanged through shared memory.
 // Intermediate operands go back to shared memory as bf16 rows in the 128-byte swizzle.
 //
@@ -34,9 +34,9 @@ namespace cvb {
 constexpr int BC = 64;
 constexpr int BD = 128;
 // Four warpgroups: warps w, w + 4, w + 8, w + 12 share TMEM lane quadrant w and split the columns of every hand-off
-// between two MMA rounds (32 of 128, 16 of 64).  One item is a serial chain of ten such stages and its 214 KB leave room
-// for one CTA per SM, so the chain's length is the kernel's time: 16 x 1280 x 16 heads took 633 us with two warpgroups,
-// 586 with four.
+// between two MMA rounds (32 of 128, 16 of 64).  One item is a serial chain of ten such stages and its 217 KB leave
+// room for one CTA per SM, so the chain's length is the kernel's time: 16 x 1280 x 16 heads took 633 us with two
+// warpgroups, 587 with four.
 constexpr int BWG = 4;
 constexpr int BTHREADS = 128 * BWG;
 

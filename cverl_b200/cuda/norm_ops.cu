@@ -144,9 +144,13 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 //   dx = dres + rstd * (g - xhat * mean(g * xhat)),  g = dy * (w0 + w) [* silu(z)]
 //   dw += sum_rows dy [* silu(z)] * xhat ;  dz = dy * xhat * (w0+w) * silu'(z)
 // ---------------------------------------------------------------------------
-// Rows of up to 1024 elements: x, dy, the residual gradient (and the gate) of ROWS rows are loaded together, stay packed
-// in registers between the dot product and the result, so a row costs one memory latency.  Reading them again for the second half, and the residual gradient only there, made it two: 40,960
-// rows of 1024 with a residual gradient took 138 us, 82 now (5.1 TB/s).
+// Rows of up to 1024 elements: x, dy, the residual gradient (and the gate) of ROWS rows are loaded together and stay
+// packed in registers between the dot product and the result, so a row costs one memory latency.  Reading them again
+// for the second half, and the residual gradient only there, made it two: 40,960 rows of 1024 with a residual gradient
+// (336 MB read and written) took 138 us, 84 now (4.0 TB/s, 0.62 of the copy rate: two blocks per SM, whose warps load
+// and compute in turn).  ROWS is what fits beside NVEC x 8 sums of dw in 128 registers: ROWS x NVEC is 4 without a gate
+// and 2 with one, or a single row where NVEC alone is as much (three operands of NVEC pieces, 48 registers; a gated row
+// of 1024 is 64 and spills 34 bytes).
 template <int NVEC, int ROWS, bool GATE>
 __global__ void __launch_bounds__(NORM_THREADS, 2)
 rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
@@ -749,13 +753,15 @@ extern "C" int cvb_rmsnorm_fwd(const void* x, const void* resid_in, const void* 
   return static_cast<int>(cudaGetLastError());
 }
 
-// KERNEL on as many blocks as are resident at once, at most one per eight groups of `group` rows
+// KERNEL on as many blocks as are resident at once, at most one per eight groups of `group` rows.  The count is taken
+// once: it only sizes the grid, and it is the same on every sm_100a device (registers bound it; of the widths that
+// share a kernel the widest asks for 1 KB of shared memory).
 template <auto KERNEL, typename... Args>
 static void norm_bwd_launch(int group, int per_sm_env, long long rows, int D, void* stream, Args... args) {
   static const int resident = [D] {
     int n = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, NORM_THREADS, D * sizeof(float)) == cudaSuccess && n > 0
-               ? n : 1;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, NORM_THREADS, D * sizeof(float));
+    return e == cudaSuccess && n > 0 ? n : 1;
   }();
   const int grid = min(norm_grid(rows, group), 148 * (per_sm_env > 0 ? per_sm_env : resident));
   KERNEL<<<grid, NORM_THREADS, D * sizeof(float), static_cast<cudaStream_t>(stream)>>>(args...);
@@ -782,10 +788,14 @@ extern "C" int cvb_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
       static_cast<const __nv_bfloat16*>(dres), static_cast<__nv_bfloat16*>(dx),                             \
       static_cast<__nv_bfloat16*>(dgate), dw, rows, D, x_stride, gate_stride, dx_stride, w_offset,          \
       gate_block, gate_block_stride, dgate_stride, dgate_block_stride
-#define CVB_BWD_ROWS(NV, RW, RG)                                                                               \
+#define CVB_BWD_ROWS(NV, RW, RG)                                                                            \
   case NV:                                                                                                  \
-    if (gate) norm_bwd_launch<rmsnorm_bwd_rows_kernel<NV, RG, true>>(32 / lanes * RG, per_sm_env, rows, D, stream, CVB_BWD_ARGS); \
-    else norm_bwd_launch<rmsnorm_bwd_rows_kernel<NV, RW, false>>(32 / lanes * RW, per_sm_env, rows, D, stream, CVB_BWD_ARGS);     \
+    if (gate)                                                                                               \
+      norm_bwd_launch<rmsnorm_bwd_rows_kernel<NV, RG, true>>(32 / lanes * RG, per_sm_env, rows, D, stream,  \
+                                                             CVB_BWD_ARGS);                                 \
+    else                                                                                                    \
+      norm_bwd_launch<rmsnorm_bwd_rows_kernel<NV, RW, false>>(32 / lanes * RW, per_sm_env, rows, D, stream, \
+                                                              CVB_BWD_ARGS);                                \
     break;
 #define CVB_BWD(NV)                                                                                         \
   case NV:                                                                                                  \

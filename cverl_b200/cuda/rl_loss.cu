@@ -239,7 +239,8 @@ struct PpoArgs {
 struct PpoSums {
   double loss = 0, clip = 0, kl = 0, low = 0, ref = 0;
 };
-__device__ __forceinline__ void ppo_token(const PpoArgs& a, long long i, double msum, double nseq, float cnt, PpoSums& s) {
+__device__ __forceinline__ void ppo_token(const PpoArgs& a, long long i, double msum, double nseq, float cnt,
+                                          PpoSums& s) {
   const float m = a.mask[i];
   const float A = a.adv[i];
   const float draw = a.lp[i] - a.old_lp[i];
@@ -323,12 +324,20 @@ __global__ void ppo_finalize_kernel(const double* ws, float* out) {
 }
 
 // --------------------------- small batches: one launch ----------------------
-// Up to RL_SMALL_N tokens the launches are the time: 64 x 512 took 4 for the loss and 3 for the advantage, 50 us a pass on
-// the host's side for 15 us of kernels; one launch each makes it 38.  One cluster of eight CTAs does all passes: row sums
-// by warp, tokens by thread, sums go from CTA to CTA through distributed shared memory, and the cluster barrier takes the
-// place of the next launch.  The limits: eight SMs fall behind on the 64-bit sums of the loss (64 x 512: 11.6 us against
-// 8.9 in four launches, 128 x 1024: 22.8 against 12), and on the comparison of every row with every row in the advantage
-// (64 rows: 5.7 us against 5.8, 2,048 rows: 66 against 11).
+// One launch each for the loss (three and a memset otherwise) and the advantage (three).  One cluster of eight CTAs
+// does all passes: row sums by warp, tokens by thread, sums go from CTA to CTA through distributed shared memory, and
+// the cluster barrier takes the place of the next launch.  Bound by the launch and the barriers on the device, by the host
+// around it: both calls on 64 x 512 take 37.6 us a pass, 47.6 before.
+// The limit of the loss is the size up to which the device is not slower either (eight SMs fall behind on the 64-bit
+// sums); us a call on the device / from call to result / on a busy host, one launch against three:
+//     8,192 tokens (16 x 512)   8.3, 10.3 / 23.9, 25.3 / 10.3, 15.4
+//    32,768        (64 x 512)  10.5, 10.2 / 26.0, 25.5 / 12.4, 15.3
+//                 (256 x 128)  10.2, 11.2 / 25.9, 26.6 / 12.3, 15.4
+//    49,152        (96 x 512)  12.0, 10.8 / 27.7, 26.6 / 14.4, 15.4
+//   131,072       (256 x 512)  19.8, 13.1 / 35.4, 29.4 / 22.6, 17.1
+// The advantage compares every row with every row, which eight SMs do up to 256 rows in the time of the launches saved:
+// 256 x 128 5.3, 5.6 / 18.8, 23.2 / 8.5, 12.9; 32 x 1024 (long rows, one warp each) 7.7, 5.6 / 21.9, 23.4 / 10.3, 12.8;
+// 512 x 32 9.2, 6.1 / 23.3, 23.7 / 10.3, 12.9; 1,024 x 32 22.0, 7.2 / 36.4, 25.9 / 24.6, 14.3.
 constexpr int RL_CLUSTER = 8;
 constexpr int RL_SMALL_THREADS = 1024;
 constexpr long long RL_SMALL_N = 32768;
@@ -370,8 +379,8 @@ ppo_loss_small_kernel(const PpoArgs a, float* rowcnt, float* __restrict__ out) {
   const unsigned n = static_cast<unsigned>(a.rows * a.cols);   // <= RL_SMALL_N
   for (unsigned i = cluster.block_rank() * RL_SMALL_THREADS + threadIdx.x; i < n; i += RL_CLUSTER * RL_SMALL_THREADS)
     ppo_token(a, i, msum, nseq, a.agg_mode == 0 ? 0.f : __ldcg(rowcnt + i / static_cast<unsigned>(a.cols)), s);
-  const double sums[5] = {block_sum_d(s.loss, sh), block_sum_d(s.clip, sh), block_sum_d(s.kl, sh), block_sum_d(s.low, sh),
-                          block_sum_d(s.ref, sh)};
+  const double sums[5] = {block_sum_d(s.loss, sh), block_sum_d(s.clip, sh), block_sum_d(s.kl, sh),
+                          block_sum_d(s.low, sh), block_sum_d(s.ref, sh)};
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < 5; ++k) part[2 + k] = sums[k];
@@ -387,8 +396,8 @@ ppo_loss_small_kernel(const PpoArgs a, float* rowcnt, float* __restrict__ out) {
 
 __global__ void __cluster_dims__(RL_CLUSTER, 1, 1) __launch_bounds__(RL_SMALL_THREADS)
 grpo_small_kernel(const float* __restrict__ rewards, const float* __restrict__ mask, const long long* __restrict__ gid,
-                  float eps, int norm_by_std, float* __restrict__ adv, float* __restrict__ ret, float* scores, long long rows,
-                  int cols) {
+                  float eps, int norm_by_std, float* __restrict__ adv, float* __restrict__ ret, float* scores,
+                  long long rows, int cols) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int lane = threadIdx.x & 31;
@@ -494,7 +503,7 @@ extern "C" int cvb_ppo_loss(const float* old_lp, const float* lp, const float* a
 }
 
 // ---------------------- GRPO advantage without allocation -------------------
-// Same three kernels as cvb_grpo_advantage; the 2*rows floats of per-row scratch (row scores,
+// The three kernels of a cvb_grpo_advantage call above its one-launch limit; the 2*rows floats of scratch (row scores,
 // then per-row scalars) come from a fixed array in this library's device image, so neither the
 // caller nor this function allocates.  See rl_no_alloc.h for who needs that and for the rules.
 #include <cstdio>

@@ -23,11 +23,12 @@ def _enabled() -> bool:
 def supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, seq: int) -> bool:
     """bf16, head dim 128 or 256, sequence length a multiple of 128.
 
-    The kernels take any length, but no rule on the length alone makes them the faster side at the others, and a rule on the
-    batch as well would give a sequence other roundings in a small batch than in a large one (old log-probabilities scored
-    at one micro-batch size, new ones formed at another).  8 / 2 heads of 256, forward and backward: 8 x 1088 704 us in the
-    library and 419 here, but 1 x 1225 200 and 333, 1 x 2500 545 and 633, since a key block's CTA walks the queries of a
-    whole GQA group; head dim 128, 32 / 4 heads: 4 x 1500 467 in the library, 4 x 1536 660 here."""
+    The kernels take any length, but at other lengths no rule on the length alone makes them the faster side, and a
+    rule on the batch would give a sequence other roundings in a small batch than in a large one (old log-probabilities
+    scored at one micro-batch size, new ones formed at another).  Forward and backward, 8 / 2 heads of 256: 8 x 1088
+    takes 704 us in the library and 419 here, but 1 x 1225 takes 200 and 333 and 1 x 2500 545 and 633, since one CTA
+    walks the queries of a whole GQA group.  32 / 4 heads of 128: 4 x 1500 takes 467 in the library, 4 x 1536 here 660.
+    """
     if not (_enabled() and q.is_cuda and q.dtype == k.dtype == v.dtype == torch.bfloat16):
         return False
     d = q.shape[-1]

@@ -72,7 +72,8 @@ def test_ragged_calls_keep_the_transforms_of_the_general_path():
     from cverl_b200.ops import attention
     (q, k), seq = _qk(3, 1001), 1001
     one = attention.causal_attention(q, k, k, 3, seq)
-    two = torch.func.vmap(lambda a, b: attention.causal_attention(a, b, b, 3, seq))(torch.stack([q, q]), torch.stack([k, k]))
+    two = torch.func.vmap(lambda a, b: attention.causal_attention(a, b, b, 3, seq))(torch.stack([q, q]),
+                                                                                     torch.stack([k, k]))
     # bf16 results of the same sums, in another order if the library splits the larger batch differently
     assert (two.float() - one.float()).norm() <= 2 ** 0.5 * 2.0 ** -8 * one.float().norm()
     dq = torch.func.grad(lambda a: attention.causal_attention(a, k, k, 3, seq).float().sum())(q)

@@ -57,7 +57,7 @@ def test_expert_block_matches_a_loop_over_experts(T, E, k, H, inter, one, main_g
 
 @pytest.mark.parametrize("layout", ["strided", "misaligned"])
 def test_expert_block_copies_rows_that_cannot_be_read_in_place(layout):
-    """Token rows and output gradients with a row stride, or 2 bytes off a 16-byte boundary, give what packed ones give."""
+    """Token rows and output gradients with a row stride, or 2 bytes off a 16-byte boundary: the result of packed ones."""
     from cverl_b200 import _native as nv
     from cverl_b200.ops.moe import moe_experts, supported
     g = torch.Generator(device="cuda").manual_seed(3)

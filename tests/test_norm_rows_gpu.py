@@ -24,8 +24,9 @@ def _shapes(small, above):
     return [s for group in small for s in group] + above
 
 
-@pytest.mark.parametrize("D,rows", _shapes([[(D, r) for r in (1, 3, 9, 70, 1000)] for D in (64, 128, 256, 512, 768, 1024, 1280)],
-                                           [(64, 120_003), (256, 40_961), (768, 9_001), (1024, 9_001), (1024, 40_961)]))
+@pytest.mark.parametrize("D,rows", _shapes(
+    [[(D, r) for r in (1, 3, 9, 70, 1000)] for D in (64, 128, 256, 512, 768, 1024, 1280)],
+    [(64, 120_003), (256, 40_961), (768, 9_001), (1024, 9_001), (1024, 40_961)]))
 @pytest.mark.parametrize("resid", [False, True])
 def test_add_rmsnorm_backward(D, rows, resid):
     from cverl_b200 import ops

@@ -12,7 +12,8 @@ def test_counted_launches(rows, cols, loss, adv):
     from cverl_b200.ops import rl
     x, mask = torch.randn(rows, cols, device="cuda"), torch.ones(rows, cols, device="cuda")
     groups = torch.arange(rows, device="cuda") // 4
-    for fn, want in ((lambda: rl.fused_ppo_loss(x, x, x, mask), loss), (lambda: rl.fused_grpo_advantage(x, mask, groups), adv)):
+    for fn, want in ((lambda: rl.fused_ppo_loss(x, x, x, mask), loss),
+                     (lambda: rl.fused_grpo_advantage(x, mask, groups), adv)):
         n = ops.launch_counter["n"]
         fn()
         assert ops.launch_counter["n"] - n == want
